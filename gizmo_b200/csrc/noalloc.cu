@@ -7,14 +7,17 @@
 // gz_context, which allocates its buffers. This entry point computes the same
 // fixed-h density sums as gz_density_sums for a particle set that the caller
 // already holds in device memory, and allocates nothing: its only scratch is
-// the packed neighbour-record array below, a file-scope device array of
-// kMaxParticles records (4 MiB) that every GPU loading this library holds
-// until the process exits.
+// the static Scratch below (3.2 MiB of device memory) that every GPU loading this
+// library holds until the process exits.
 //
-// The neighbour loop is all-pairs (the set is small by construction), tiled
-// through shared memory; the pair arithmetic is the one of k_density_sums in
-// FP64 (this file is built with -fmad=false like passes_fp64.cu), so the sums
-// agree with gz_density_sums up to summation order.
+// The particles are put in Morton order first, so that runs of 32 have small
+// bounding boxes; a run of 32 targets then tests every other run's box and only
+// scans the particles of the runs it can reach. Each pair of those is screened in
+// FP32, with a margin that bounds the FP32 rounding, and only the pairs near or
+// inside the support take the exact FP64 test and the sums, whose arithmetic is
+// the one of k_density_sums in FP64 (this file is built with -fmad=false like
+// passes_fp64.cu), so the sums agree with gz_density_sums up to summation order.
+#include <cub/cub.cuh>
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -27,125 +30,364 @@ using namespace gz;
 namespace {
 
 constexpr int kMaxParticles = GZ_NOALLOC_MAX_PARTICLES;
-constexpr int kTile = 128;
+constexpr int kRun = 32;      // particles of a run: the targets of a block, and the unit of the box tests
+constexpr int kSlices = 8;    // warps of a block, each taking its share of the candidates for the block's targets
+constexpr int kShare = kRun / kSlices;  // candidates a warp takes from each run
+constexpr int kHits = 32;     // screened candidates a lane holds before the warp evaluates them
+constexpr int kFewHits = 8;   // up to as many of a target are evaluated by its own lane
+constexpr int kKeyBits = 24;  // Morton key, 8 bits an axis: three 8-bit radix passes
 constexpr int kMaxDevices = 128;
+constexpr size_t kSortBytes = 1 << 20;
+static_assert(kMaxParticles <= 65536, "a hit is a 16-bit particle index");
 
-// The only scratch of the entry point: one packed record per particle of the
-// current call. Shared by every call on a device; fully rewritten by each call
-// for the particles it covers, so nothing in it needs clearing.
-static __device__ __align__(256) DensRec g_records[kMaxParticles];
+// Bounding box of a run, rounded outward to FP32: lo.w the largest coordinate
+// magnitude, hi.w the largest |h|. A run that holds a NaN is given the whole space.
+struct RunBox {
+    float4 lo, hi;
+};
+
+// The only scratch of the entry point. Shared by every call on a device; what a
+// call reads it has written itself, so nothing in it needs clearing.
+struct Scratch {
+    unsigned key[2][kMaxParticles];
+    int order[2][kMaxParticles];              // sorted -> caller's index: [1] after the sort
+    float4 pos[kMaxParticles];                // sorted FP32 positions; w: the caller's index
+    RunBox box[kMaxParticles / kRun];
+    unsigned char sort[kSortBytes];           // temporary storage of the radix sort
+};
+static __device__ __align__(256) Scratch g_scratch;
 
 std::mutex g_setup_mutex;
-DensRec *g_records_ptr[kMaxDevices] = {};  // device address of g_records, per device
+Scratch *g_scratch_ptr[kMaxDevices] = {};  // device address of g_scratch, per device
 
-__global__ void k_noalloc_pack(int n, const double *__restrict__ pos, const double *__restrict__ vel,
-                               const double *__restrict__ mass, DensRec *rec)
+// What the sums read of the scratch.
+struct SumsWork {
+    const int *order;
+    const float4 *pos;
+    const RunBox *box;
+};
+
+__device__ unsigned spread8(unsigned x)
+{
+    x = (x | (x << 8)) & 0x00f00fu;
+    x = (x | (x << 4)) & 0x0c30c3u;
+    return (x | (x << 2)) & 0x249249u;
+}
+
+__global__ void k_noalloc_keys(int n, const double *__restrict__ pos, double box, unsigned *key, int *order)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    DensRec r;
-    r.x = pos[3 * (size_t)i]; r.y = pos[3 * (size_t)i + 1]; r.z = pos[3 * (size_t)i + 2];
-    r.m = mass[i];
-    r.vx = vel[3 * (size_t)i]; r.vy = vel[3 * (size_t)i + 1]; r.vz = vel[3 * (size_t)i + 2];
-    r.pad = 0.0;
-    rec[i] = r;
+    unsigned k = 0;
+    for (int c = 0; c < 3; c++) {  // (the order only has to be good: coordinates outside the box are clamped)
+        const double v = pos[3 * (size_t)i + c] / box * 256.0;
+        k |= spread8(v > 0.0 ? (v < 255.0 ? (unsigned)v : 255u) : 0u) << c;
+    }
+    key[i] = k;
+    order[i] = i;
 }
 
-// One thread per target; every particle of the set is a candidate, streamed
-// through shared memory kTile records at a time and accepted on r^2 < h^2
-// (DensitySpec::pair_kernel, density_loop.h:1140-1385).
-__global__ void __launch_bounds__(kTile) k_noalloc_density_sums(PassParams p, int n, const double *__restrict__ pos,
-                                                                 const double *__restrict__ vel,
-                                                                 const double *__restrict__ hs,
-                                                                 const DensRec *__restrict__ rec, double *acc,
-                                                                 double *pv)
+__global__ void __launch_bounds__(128) k_noalloc_runs(int n, const double *__restrict__ pos,
+                                                      const double *__restrict__ hs, const int *__restrict__ order,
+                                                      float4 *out, RunBox *box)
 {
-    __shared__ DensRec tile[kTile];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < n;
-    double xi = 0, yi = 0, zi = 0, hd = 0, vix = 0, viy = 0, viz = 0;
-    if (valid) {
-        xi = pos[3 * (size_t)i]; yi = pos[3 * (size_t)i + 1]; zi = pos[3 * (size_t)i + 2];
-        vix = vel[3 * (size_t)i]; viy = vel[3 * (size_t)i + 1]; viz = vel[3 * (size_t)i + 2];
-        hd = hs[i];
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const float inf = __int_as_float(0x7f800000);
+    float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf}, mag = 0.0f, h = 0.0f;
+    bool nan = false;
+    if (s < n) {
+        const size_t o = (size_t)order[s];
+        const double hv = fabs(hs[o]);
+        float f[3];
+        for (int c = 0; c < 3; c++) {
+            const double v = pos[3 * o + c];
+            f[c] = __double2float_rn(v);
+            lo[c] = __double2float_rd(v);
+            hi[c] = __double2float_ru(v);
+            mag = fmaxf(mag, __double2float_ru(fabs(v)));
+            nan |= v != v;
+        }
+        nan |= hv != hv;
+        h = __double2float_ru(hv);
+        out[s] = make_float4(f[0], f[1], f[2], __int_as_float((int)o));
     }
-    const double h2 = hd * hd;
-    double hinv = 0, hinv3 = 0, hinv4 = 0;
-    if (valid) k_hinv(hd, hinv, hinv3, hinv4);
+    for (int d = 16; d > 0; d >>= 1) {
+        for (int c = 0; c < 3; c++) {
+            lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], d));
+            hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], d));
+        }
+        mag = fmaxf(mag, __shfl_xor_sync(0xffffffffu, mag, d));
+        h = fmaxf(h, __shfl_xor_sync(0xffffffffu, h, d));
+    }
+    nan = __any_sync(0xffffffffu, nan);
+    if ((threadIdx.x & 31) == 0 && s < n) {
+        box[s / kRun] = nan ? RunBox{make_float4(-inf, -inf, -inf, mag), make_float4(inf, inf, inf, inf)}
+                            : RunBox{make_float4(lo[0], lo[1], lo[2], mag), make_float4(hi[0], hi[1], hi[2], h)};
+    }
+}
+
+// The most by which an FP32 separation can differ from the FP64 one, for
+// coordinates of magnitude up to m: each axis rounds two coordinates (2^-24 m
+// each), their difference (2^-24 2m) and the wrap (2^-24 (2m + box)), in all less
+// than 2^-24 (8m + 2 box) an axis and, over three axes and the rounding of the
+// squares, less than 2^-24 (16m + 8 box).
+__device__ __forceinline__ float screen_margin(float m, float box) { return 5.9604645e-8f * (16.0f * m + 8.0f * box); }
+
+// distance of the interval [a, b] of coordinate differences to the nearest of 0 and +-box, where a pair's
+// minimum image on one axis is measured from
+__device__ __forceinline__ float axis_distance(float a, float b, float box)
+{
+    const float d0 = fmaxf(a, -b), dp = fmaxf(a - box, box - b), dm = fmaxf(a + box, -box - b);
+    return fmaxf(fminf(d0, fminf(dp, dm)), 0.0f);
+}
+
+struct Target {
+    double x, y, z, vx, vy, vz, h2, hinv;
+};
+
+struct SumsInput {
+    const double *pos, *vel, *mass;
+};
+
+// one neighbour's contribution: DensitySpec::pair_kernel (density_loop.h:1140-1385)
+__device__ __forceinline__ void add_pair(const PassParams &p, const SumsInput &in, const Target &t, size_t j, double *a)
+{
+    const double mj = in.mass[j], xj = in.pos[3 * j], yj = in.pos[3 * j + 1], zj = in.pos[3 * j + 2];
+    const double vjx = in.vel[3 * j], vjy = in.vel[3 * j + 1], vjz = in.vel[3 * j + 2];  // all in flight together
+    if (mj <= 0) return;
+    double dx, dy, dz;
+    const double r2 = sep2(t.x, t.y, t.z, xj, yj, zj, p.box, p.half, dx, dy, dz);
+    if (r2 >= t.h2) return;
     const int mfv = p.method == 1;
+    const double hinv3 = t.hinv * t.hinv * t.hinv, hinv4 = hinv3 * t.hinv;  // as k_hinv
+    const double r = sqrt(r2);
+    const double u = r * t.hinv;
+    double wk, dwk;
+    k_main(p.kernel, u, hinv3, hinv4, wk, dwk);
+    const double mj_wk = mj * wk;
+    a[0] += wk;
+    a[1] += mj_wk;
+    if (mfv && r == 0.0) {
+        a[14] += mj_wk * vjx;
+        a[15] += mj_wk * vjy;
+        a[16] += mj_wk * vjz;
+    }
+    a[2] += -(3.0 * t.hinv * wk + u * dwk);
+    if (r > 0.0) {
+        a[4] += dx * dx * wk;
+        a[5] += dy * dy * wk;
+        a[6] += dz * dz * wk;
+        a[7] += dx * dy * wk;
+        a[8] += dy * dz * wk;
+        a[9] += dx * dz * wk;
+        a[10] += wk * dx;
+        a[11] += wk * dy;
+        a[12] += wk * dz;
+        const double dvx = t.vx - vjx, dvy = t.vy - vjy, dvz = t.vz - vjz;
+        if (mfv) {
+            a[14] += mj_wk * (t.vx - dvx);
+            a[15] += mj_wk * (t.vy - dvy);
+            a[16] += mj_wk * (t.vz - dvz);
+        }
+        a[3] -= dwk * (dx * dvx + dy * dvy + dz * dvz) / r;
+    }
+}
+
+// One target per lane: a block holds the 32 targets of a run. Its warps first test
+// the boxes of all runs and list the ones the targets can reach; then each warp
+// takes kShare candidates of every listed run (so the work, which is concentrated
+// in the few nearest runs, is spread over the warps) and screens 32 candidates at
+// a time: a broadcast shared-memory read and ~14 FP32 instructions a pair, no
+// branch, the outcomes the bits of a mask. The candidates that pass are collected
+// in shared memory and evaluated together, so the FP64 arithmetic runs with most
+// lanes busy although few of the scanned pairs need it; the warps' sums are added
+// at the end in a fixed order. A pair is rejected only when its FP32 separation is
+// beyond |h| by more than the margin; NaNs are never rejected.
+//
+// What bounds it: the latency of a block's chain (run list, screen, evaluation),
+// not throughput. Measured on a clustered MFV set (whole call, the five launches
+// of the sort included): 57, 250 and 459 us at 1,000, 20,000 and 65,536 particles,
+// against 467, 5,731 and 18,294 us with one thread per target testing every pair
+// in FP64 (157 blocks of 128 at 20,000: four warps per multiprocessor, each
+// taking the sums for one or two of its lanes at a time). Four warps a block: 82,
+// 332, 544 us; eight at three blocks per multiprocessor (80 registers, spills):
+// 66, 292, 514 us. All pairs screened, without the order and the boxes: 27, 404
+// and 2,803 us.
+__global__ void __launch_bounds__(32 * kSlices, 2) k_noalloc_density_sums(PassParams p, int n,
+                                                                          const double *__restrict__ pos,
+                                                                          const double *__restrict__ vel,
+                                                                          const double *__restrict__ mass,
+                                                                          const double *__restrict__ hs, SumsWork w,
+                                                                          double *acc, double *pv)
+{
+    constexpr int kThreads = 32 * kSlices;
+    // the scan's tiles and hits, then (in the same place) the slices' sums
+    struct Scan {
+        float4 tile[kSlices][32];
+        unsigned short hit[kHits][kThreads];
+    };
+    __shared__ union {
+        Scan scan;
+        double sum[kSlices][17][32];
+    } sh;
+    __shared__ unsigned short s_run[kMaxParticles / kRun];  // the reached runs, ascending
+    __shared__ int s_cnt[kSlices];
+    __shared__ unsigned s_top;  // largest coordinate magnitude among them
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const int s = blockIdx.x * kRun + lane;
+    const bool valid = s < n;
+    const int sv = valid ? s : n - 1;  // a lane past the end follows the last target and stores nothing
+    const size_t i = (size_t)w.order[sv];
+    Target me;
+    me.x = pos[3 * i]; me.y = pos[3 * i + 1]; me.z = pos[3 * i + 2];
+    me.vx = vel[3 * i]; me.vy = vel[3 * i + 1]; me.vz = vel[3 * i + 2];
+    const double hd = hs[i];
+    me.h2 = hd * hd;
+    double hinv3, hinv4;
+    k_hinv(hd, me.hinv, hinv3, hinv4);
     double a[17];
 #pragma unroll
     for (int k = 0; k < 17; k++) a[k] = 0;
-    for (int t0 = 0; t0 < n; t0 += kTile) {
-        if (t0 + (int)threadIdx.x < n) tile[threadIdx.x] = rec[t0 + threadIdx.x];
-        __syncthreads();
-        const int m = min(kTile, n - t0);
-        if (valid) {
-            for (int k = 0; k < m; k++) {
-                const DensRec rj = tile[k];
-                if (rj.m <= 0) continue;
-                double dx, dy, dz;
-                const double r2 = sep2(xi, yi, zi, rj.x, rj.y, rj.z, p.box, p.half, dx, dy, dz);
-                if (r2 >= h2) continue;
-                const double r = sqrt(r2);
-                const double u = r * hinv;
-                double wk, dwk;
-                k_main(p.kernel, u, hinv3, hinv4, wk, dwk);
-                const double mj_wk = rj.m * wk;
-                a[0] += wk;
-                a[1] += mj_wk;
-                if (mfv && r == 0.0) {
-                    a[14] += mj_wk * rj.vx;
-                    a[15] += mj_wk * rj.vy;
-                    a[16] += mj_wk * rj.vz;
-                }
-                a[2] += -(3.0 * hinv * wk + u * dwk);
-                if (r > 0.0) {
-                    a[4] += dx * dx * wk;
-                    a[5] += dy * dy * wk;
-                    a[6] += dz * dz * wk;
-                    a[7] += dx * dy * wk;
-                    a[8] += dy * dz * wk;
-                    a[9] += dx * dz * wk;
-                    a[10] += wk * dx;
-                    a[11] += wk * dy;
-                    a[12] += wk * dz;
-                    const double dvx = vix - rj.vx, dvy = viy - rj.vy, dvz = viz - rj.vz;
-                    if (mfv) {
-                        a[14] += mj_wk * (vix - dvx);
-                        a[15] += mj_wk * (viy - dvy);
-                        a[16] += mj_wk * (viz - dvz);
-                    }
-                    a[3] -= dwk * (dx * dvx + dy * dvy + dz * dvz) / r;
-                }
+
+    // The collected candidates. Usually every lane evaluates its own; a target
+    // that holds far more than the others (a long kernel that reaches into a
+    // clump) would keep one lane busy and the rest idle, so the warp evaluates
+    // its candidates together, one per lane, and adds the sums across the lanes.
+    int hits = 0;
+    const SumsInput in{pos, vel, mass};
+    auto evaluate = [&]() {
+        unsigned many = __ballot_sync(full, hits > kFewHits);
+        // (in units of a lane's own evaluation: a shared one costs about three with its cross-lane sums)
+        if (__popc(many) * 3 > __reduce_max_sync(full, hits) - kFewHits) many = 0u;
+        for (; many; many &= many - 1u) {
+            const int tl = __ffs(many) - 1;
+            Target t;
+            t.x = __shfl_sync(full, me.x, tl); t.y = __shfl_sync(full, me.y, tl); t.z = __shfl_sync(full, me.z, tl);
+            t.vx = __shfl_sync(full, me.vx, tl); t.vy = __shfl_sync(full, me.vy, tl); t.vz = __shfl_sync(full, me.vz, tl);
+            t.h2 = __shfl_sync(full, me.h2, tl); t.hinv = __shfl_sync(full, me.hinv, tl);
+            double b[17];
+#pragma unroll
+            for (int k = 0; k < 17; k++) b[k] = 0;
+            if (lane < __shfl_sync(full, hits, tl)) add_pair(p, in, t, sh.scan.hit[lane][(threadIdx.x & ~31) + tl], b);
+#pragma unroll
+            for (int k = 0; k < 17; k++) {
+                const double v = warp_sum(b[k], full, 32);
+                if (lane == tl) a[k] += v;
             }
+            if (lane == tl) hits = 0;
+        }
+        const int most = __reduce_max_sync(full, hits);
+        for (int k = 0; k < most; k++)
+            if (k < hits) add_pair(p, in, me, sh.scan.hit[k][threadIdx.x], a);
+        hits = 0;
+        __syncwarp();
+    };
+
+    const float4 mf = w.pos[sv];
+    const RunBox mine = w.box[blockIdx.x];
+    const float boxf = (float)p.box, hf = __double2float_ru(fabs(hd));
+    const int runs = (n + kRun - 1) / kRun;
+    // the runs the targets can reach
+    if (threadIdx.x == 0) s_top = 0u;
+    int reached = 0;
+    for (int q0 = 0; q0 < runs; q0 += kThreads) {
+        const int q = q0 + (int)threadIdx.x;
+        bool in = false;
+        float top = 0.0f;
+        if (q < runs) {
+            const RunBox b = w.box[q];
+            top = b.lo.w;
+            const float R = mine.hi.w + screen_margin(fmaxf(mine.lo.w, top), boxf);
+            const float gx = axis_distance(mine.lo.x - b.hi.x, mine.hi.x - b.lo.x, boxf);
+            const float gy = axis_distance(mine.lo.y - b.hi.y, mine.hi.y - b.lo.y, boxf);
+            const float gz = axis_distance(mine.lo.z - b.hi.z, mine.hi.z - b.lo.z, boxf);
+            in = !(gx * gx + gy * gy + gz * gz > R * R * 1.000001f);
+        }
+        const unsigned bal = __ballot_sync(full, in);
+        const unsigned tmax = __reduce_max_sync(full, in ? __float_as_uint(top) : 0u);
+        __syncthreads();  // s_cnt of the last round has been read
+        if (lane == 0) {
+            s_cnt[slice] = __popc(bal);
+            if (bal) atomicMax(&s_top, tmax);  // (magnitudes are not negative: their bits order like them)
         }
         __syncthreads();
-    }
-    if (!valid) return;
+        int at = reached;
 #pragma unroll
-    for (int k = 0; k < 13; k++) acc[14 * (size_t)i + k] = a[k];
-    acc[14 * (size_t)i + 13] = 0.0;
-    if (pv)
-        for (int k = 0; k < 3; k++) pv[3 * (size_t)i + k] = a[14 + k];
+        for (int k = 0; k < kSlices; k++) {
+            if (k < slice) at += s_cnt[k];
+            reached += s_cnt[k];
+        }
+        if (in) s_run[at + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)q;
+    }
+    __syncthreads();
+    const float hi = hf + screen_margin(fmaxf(__uint_as_float(s_top), mine.lo.w), boxf);
+    const float hi2 = hi * hi * 1.000001f;
+    for (int q0 = 0; q0 < reached; q0 += kSlices) {
+        const int ql = q0 + lane / kShare;
+        int c = n;
+        if (ql < reached) c = s_run[ql] * kRun + slice * kShare + lane % kShare;
+        const unsigned have = __ballot_sync(full, c < n);
+        if (c < n) sh.scan.tile[slice][lane] = w.pos[c];
+        __syncwarp();
+        unsigned pass = 0;
+#pragma unroll
+        for (int k = 0; k < 32; k++) {
+            const float4 q = sh.scan.tile[slice][k];
+            // the minimum image's magnitude: |d|, or box - |d| beyond half the box (squared below)
+            float dx = fabsf(mf.x - q.x), dy = fabsf(mf.y - q.y), dz = fabsf(mf.z - q.z);
+            dx = fminf(dx, boxf - dx);
+            dy = fminf(dy, boxf - dy);
+            dz = fminf(dz, boxf - dz);
+            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            if (!(r2 > hi2)) pass |= 1u << k;
+        }
+        pass &= have;
+        while (__any_sync(full, pass != 0u)) {
+            if (pass) {
+                const int k = __ffs(pass) - 1;
+                sh.scan.hit[hits++][threadIdx.x] = (unsigned short)__float_as_int(sh.scan.tile[slice][k].w);
+                pass &= pass - 1u;
+            }
+            __syncwarp();
+            if (__any_sync(full, hits == kHits)) evaluate();
+        }
+        __syncwarp();  // the tile has been read
+    }
+    evaluate();
+
+    // the slices' sums, added in slice order, one sum at a time per warp
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 17; k++) sh.sum[slice][k][lane] = a[k];
+    __syncthreads();
+    for (int k = slice; k < 17; k += kSlices) {
+        double v = sh.sum[0][k][lane];
+#pragma unroll
+        for (int q = 1; q < kSlices; q++) v += sh.sum[q][k][lane];
+        if (!valid) continue;
+        if (k < 13) acc[14 * i + k] = v;
+        else if (k == 13) acc[14 * i + 13] = 0.0;
+        else if (pv) pv[3 * i + (k - 14)] = v;
+    }
 }
 
-// Device address of g_records on the current device, looked up once per
-// device (host code must not pass the symbol itself: on the host it names a
-// stand-in, not device memory).
-int records_address(DensRec **out)
+// Device address of g_scratch on the current device, looked up once per device
+// (host code must not pass the symbol itself: on the host it names a stand-in,
+// not device memory).
+int scratch_address(Scratch **out)
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return GZ_ERR_NO_DEVICE;
     if (dev < 0 || dev >= kMaxDevices) return GZ_ERR_ARG;
     std::lock_guard<std::mutex> lock(g_setup_mutex);
-    if (!g_records_ptr[dev]) {
-        void *p = nullptr;
-        const cudaError_t e = cudaGetSymbolAddress(&p, g_records);
-        if (e != cudaSuccess || !p) return GZ_ERR_CUDA;
-        g_records_ptr[dev] = (DensRec *)p;
+    if (!g_scratch_ptr[dev]) {
+        void *q = nullptr;
+        const cudaError_t e = cudaGetSymbolAddress(&q, g_scratch);
+        if (e != cudaSuccess || !q) return GZ_ERR_CUDA;
+        g_scratch_ptr[dev] = (Scratch *)q;
     }
-    *out = g_records_ptr[dev];
+    *out = g_scratch_ptr[dev];
     return GZ_OK;
 }
 
@@ -161,8 +403,8 @@ extern "C" int gz_density_sums_noalloc(const gz_params *params, int n, const dou
     if (n > kMaxParticles) return GZ_ERR_CAPACITY;
     if (n == 0) return GZ_OK;
     if (!pos || !vel || !mass || !h || !acc) return GZ_ERR_ARG;
-    DensRec *rec = nullptr;
-    const int rc = records_address(&rec);
+    Scratch *g = nullptr;
+    const int rc = scratch_address(&g);
     if (rc) return rc;
     PassParams p{};
     p.kernel = params->kernel;
@@ -177,8 +419,19 @@ extern "C" int gz_density_sums_noalloc(const gz_params *params, int n, const dou
     p.min_kernel_radius = params->min_kernel_radius;
     p.max_kernel_radius = params->max_kernel_radius;
     cudaStream_t s = (cudaStream_t)stream;
-    const unsigned blocks = (unsigned)((n + kTile - 1) / kTile);
-    k_noalloc_pack<<<blocks, kTile, 0, s>>>(n, pos, vel, mass, rec);
-    k_noalloc_density_sums<<<blocks, kTile, 0, s>>>(p, n, pos, vel, h, rec, acc, pv);
+    const unsigned blocks = (unsigned)((n + 127) / 128);
+    k_noalloc_keys<<<blocks, 128, 0, s>>>(n, pos, p.box, g->key[0], g->order[0]);
+    size_t need = 0;
+    if (cub::DeviceRadixSort::SortPairs(nullptr, need, g->key[0], g->key[1], g->order[0], g->order[1], n, 0, kKeyBits,
+                                        s) != cudaSuccess)
+        return GZ_ERR_CUDA;
+    if (need > kSortBytes) return GZ_ERR_INTERNAL;  // (0.4 MiB for the largest set)
+    if (cub::DeviceRadixSort::SortPairs(g->sort, need, g->key[0], g->key[1], g->order[0], g->order[1], n, 0, kKeyBits,
+                                        s) != cudaSuccess)
+        return GZ_ERR_CUDA;
+    k_noalloc_runs<<<blocks, 128, 0, s>>>(n, pos, h, g->order[1], g->pos, g->box);
+    const SumsWork w{g->order[1], g->pos, g->box};
+    k_noalloc_density_sums<<<(unsigned)((n + kRun - 1) / kRun), 32 * kSlices, 0, s>>>(p, n, pos, vel, mass, h, w, acc,
+                                                                                     pv);
     return cudaGetLastError() == cudaSuccess ? GZ_OK : GZ_ERR_CUDA;
 }

@@ -353,24 +353,25 @@ int gz_density_sums(gz_context *ctx, const int *active, int n_active, double *ac
  *     acc [n][14], pv [n][3] (outputs; pv may be NULL) are DEVICE pointers that
  *     the caller owns; rows follow the caller's order, every particle is a
  *     target and a candidate;
- *   - the only scratch is a static device array of GZ_NOALLOC_MAX_PARTICLES
- *     packed records (4 MiB), held by every GPU that loads the library until
- *     the process exits; n above that limit returns GZ_ERR_CAPACITY;
+ *   - the only scratch is static device memory for GZ_NOALLOC_MAX_PARTICLES
+ *     particles (3.1 MiB), held by every GPU that loads the library until the
+ *     process exits; n above that limit returns GZ_ERR_CAPACITY;
  *   - work is queued on `stream` (a cudaStream_t, NULL for the default
  *     stream) and the call returns without waiting: synchronise the stream
  *     before reading acc;
- *   - the first call on each device looks up that array's device address
+ *   - the first call on each device looks up that memory's address
  *     (a one-time set-up on the current device): make that first call before
  *     any stream capture. Under CUDA's lazy module loading (the default since
  *     CUDA 12.2) that first call is also where the library's device code is
- *     loaded on the device and the 4 MiB array is reserved, so it must come
+ *     loaded on the device and the static memory is reserved, so it must come
  *     before the caller's memory pool reserves the device; setting
  *     CUDA_MODULE_LOADING=EAGER reserves it when the process first creates
  *     its CUDA context instead. A failed set-up returns GZ_ERR_CUDA;
- *   - every call on a device uses the same array and rewrites it; two calls
+ *   - every call on a device uses the same memory and rewrites it; two calls
  *     whose work overlaps on the GPU (different streams, no ordering between
  *     them) race on it and their results are undefined.
- * The neighbour loop is all-pairs over the set, which is what bounds n. */
+ * The neighbour search takes every run of 32 particles against every other,
+ * which is what bounds n. */
 #define GZ_NOALLOC_MAX_PARTICLES 65536
 int gz_density_sums_noalloc(const gz_params *params, int n, const double *pos, const double *vel,
                             const double *mass, const double *h, double *acc, double *pv, void *stream);
