@@ -66,6 +66,7 @@ struct gz_context {
     DevBuf acc, h_built, scratch, keep, regrow, todo_a, todo_b, grow, d_beg, d_end, flag, counts, d_off, d_nbr, n_sel;
     DevBuf hmax;                     // largest kernel length the density iteration took sums at (double bits)
     DevBuf refined, rq;              // mixed form: count and queue of the force pairs evaluated again in FP64
+    DevBuf deferred, dq;             // count and queue of the force pairs left to their own kernel
     long long pairs_refined = 0;
     double h_iter_max = 0;           // ... read back after the pass
     long long d_nbr_cap = 0, d_used = 0;
@@ -291,7 +292,7 @@ std::vector<DevBuf *> all_buffers(gz_context *c)
             &c->targets, &c->targets_tmp, &c->t_node, &c->t_lo, &c->t_hi, &c->t_parent, &c->t_done, &c->t_nch,
             &c->t_cpos, &c->acc, &c->h_built, &c->scratch, &c->keep, &c->regrow, &c->todo_a, &c->todo_b, &c->grow,
             &c->d_beg, &c->d_end, &c->flag, &c->counts, &c->d_off, &c->d_nbr, &c->n_sel, &c->s_off, &c->s_nbr,
-            &c->s_counts, &c->rec, &c->work, &c->hmax, &c->refined, &c->rq, &c->pad_over, &c->pad_list, &c->pad_sum, &c->pad_counts, &c->s_acnt, &c->s_bcnt, &c->s_tmp, &c->pflux, &c->status, &c->o_vel, &c->o_mass, &c->o_u, &c->o_dt, &c->o_h, &c->o_cond, &c->dl, &c->o_timebin,
+            &c->s_counts, &c->rec, &c->work, &c->hmax, &c->refined, &c->rq, &c->deferred, &c->dq, &c->pad_over, &c->pad_list, &c->pad_sum, &c->pad_counts, &c->s_acnt, &c->s_bcnt, &c->s_tmp, &c->pflux, &c->status, &c->o_vel, &c->o_mass, &c->o_u, &c->o_dt, &c->o_h, &c->o_cond, &c->dl, &c->o_timebin,
             &c->o_vsig, &c->timebin, &c->vsig_prev, &c->wakeup, &c->binact, &c->sel_flags, &c->sel_out,
             &c->gstate, &c->g_hseed, &c->g_cseed, &c->g_over_list, &c->g_over_off, &c->g_sel,
             &c->p_stage3, &c->p_vel, &c->p_mass, &c->p_u, &c->p_dt, &c->p_h, &c->p_cond, &c->dstage,
@@ -1210,7 +1211,8 @@ int graph_buffers(gz_context *c, long long *sym_cap, long long *rq_cap, bool wit
         ensure(c, c->g_over_off, sizeof(long long) * N) || ensure(c, c->s_acnt, sizeof(int) * N) ||
         ensure(c, c->s_bcnt, sizeof(int) * N) || ensure(c, c->s_counts, sizeof(long long) * N) ||
         ensure(c, c->s_off, sizeof(long long) * (N + 1)) || ensure(c, c->refined, sizeof(unsigned long long)) ||
-        ensure(c, c->keep, N) || ensure(c, c->regrow, N) ||
+        ensure(c, c->deferred, sizeof(unsigned long long)) ||
+        ensure(c, c->dq, sizeof(RefineItem) * (size_t)deferred_cap(sc)) || ensure(c, c->keep, N) || ensure(c, c->regrow, N) ||
         ensure(c, c->g_sel, sizeof(int) * 2 * (N / kSelChunk + 1)))
         return c->err;
     // the large buffers: without room for them the pass runs plain (which
@@ -1243,6 +1245,12 @@ int graph_buffers(gz_context *c, long long *sym_cap, long long *rq_cap, bool wit
     *sym_cap = std::min<long long>({sc, (long long)(c->s_nbr.bytes / sizeof(int)), (long long)(c->s_tmp.bytes / sizeof(int)),
                                     (long long)(c->pflux.bytes / pair_flux_bytes(mixed))});
     *rq_cap = rq;
+
+// queue room for the deferred force pairs of `entries` symmetric row entries:
+// one pair in 16 (under 1 in 100 is deferred on the sets measured; when more
+// are, k_force_deferred scans the rows instead)
+long long deferred_cap(long long entries) { return std::max(65536ll, entries / 32); }
+
     return 0;
 }
 
@@ -1416,10 +1424,10 @@ int capture_gradients_force(gz_context *c, cudaStream_t s, long long rq_cap)
         GZ_CUDA(c, cudaMemsetAsync(c->refined.p, 0, sizeof(unsigned long long), s));
         const RefineQueue q{ptr<RefineItem>(c->rq), ptr<unsigned long long>(c->refined), rq_cap};
         force_mixed(c->pp, ps, ptr<int>(c->targets), n, rows, c->tpt_force, ptr<DevStatus>(c->status), c->rec.p,
-                    c->pflux.p, true, q, ptr<double>(c->acc), nullptr, s);
+                    c->pflux.p, true, q, dq, ptr<double>(c->acc), nullptr, s);
     } else {
         force_fp64(c->pp, ps, ptr<int>(c->targets), n, rows, c->tpt_force, ptr<DevStatus>(c->status), c->rec.p,
-                   c->pflux.p, true, ptr<double>(c->acc), nullptr, s);
+                   c->pflux.p, true, dq, ptr<double>(c->acc), nullptr, s);
     }
     GZ_CUDA(c, cudaGetLastError());
     return 0;
@@ -1464,6 +1472,9 @@ int graph_capture(gz_context *c, long long sym_cap, long long rq_cap, bool with_
             if ((rc = enqueue_restage(c, true))) break;
             k_g_tree_check<<<1, 1, 0, s>>>(ptr<TreeBuild>(c->t_build), ptr<GraphState>(c->gstate));
             restage_kernels = c->launches - l0 + 1 + 2 * 22 + 1 + 1;  // + tree build, bottom-up pass, check
+    GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), s));
+    const RefineQueue dq{ptr<RefineItem>(c->dq), ptr<unsigned long long>(c->deferred),
+                         (long long)(c->dq.bytes / sizeof(RefineItem))};
             if ((rc = check_last(c, "restage"))) break;
         }
         // the inputs a plain pass would restart from
@@ -1514,11 +1525,11 @@ int graph_capture(gz_context *c, long long sym_cap, long long rq_cap, bool with_
     // rows, overflow check, overflow walk, three sums instances, after_iter,
     // the selection's three steps, next; the rows' split, counts and check;
     // scatter, sort, the gradient pack and rows, the force preloop, pack,
-    // pairs, (refine,) gather, finish
+    // pairs, deferred pairs, (refine,) gather, finish
     c->g.kernels_top = 7 + restage_kernels;
     c->g.kernels_loop = 15;
     c->g.kernels_sym = 3;
-    c->g.kernels_tail = c->prm.precision == GZ_PRECISION_MIXED ? 10 : 9;
+    c->g.kernels_tail = c->prm.precision == GZ_PRECISION_MIXED ? 11 : 10;
     const cudaError_t ie = cudaGraphInstantiate(&c->g.exec, g, 0);
     if (ie != cudaSuccess) {
         char b[200];
@@ -2079,11 +2090,11 @@ int gz_hydro_force(gz_context *c, const int *active, int n_active)
                    : nullptr;
         if (mixed)
             force_mixed(c->pp, ps, ptr<int>(c->targets), na, rows, c->tpt_force, ptr<DevStatus>(c->status), c->rec.p,
-                        flux, all, q, ptr<double>(c->acc), ev, c->stream);
+                        flux, all, q, dq, ptr<double>(c->acc), ev, c->stream);
         else
             force_fp64(c->pp, ps, ptr<int>(c->targets), na, rows, c->tpt_force, ptr<DevStatus>(c->status), c->rec.p,
-                       flux, all, ptr<double>(c->acc), ev, c->stream);
-        if (na > 0) c->launches += flux ? (mixed ? 5 : 4) : 3;
+                       flux, all, dq, ptr<double>(c->acc), ev, c->stream);
+        if (na > 0) c->launches += flux ? (mixed ? 6 : 5) : 3;
         GZ_CUDA(c, cudaGetLastError());
         if (!q.item) break;
         GZ_CUDA(c, cudaMemcpyAsync(&refined, c->refined.p, sizeof(refined), cudaMemcpyDeviceToHost, c->stream));
@@ -2124,6 +2135,15 @@ int gz_set_boxes(gz_context *c, int n_boxes, const int64_t *counts)
         c->box_bits = 0;
     } else {
         for (int b = 0; b < n_boxes; b++)
+        RefineQueue dq{nullptr, nullptr, 0};
+        if (flux) {
+            if (ensure(c, c->deferred, sizeof(unsigned long long)) ||
+                ensure(c, c->dq, sizeof(RefineItem) * (size_t)deferred_cap(c->pairs_symmetric)))
+                return c->err;
+            GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), c->stream));
+            dq = RefineQueue{ptr<RefineItem>(c->dq), ptr<unsigned long long>(c->deferred),
+                             (long long)(c->dq.bytes / sizeof(RefineItem))};
+        }
             if (counts[b] < 0) return GZ_ERR_ARG;
         int bits = 0;
         while ((1 << bits) < n_boxes) bits++;

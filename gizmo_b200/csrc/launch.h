@@ -99,12 +99,14 @@ void gradients_fp64(const PassParams &p, const Particles &ps, const int *targets
 // evaluation per pair: n_entries x pair_flux_bytes. sums: 13 x n doubles of
 // scratch (the row sums before the writeback).
 // `all`: every particle is a target (flux then holds each pair once). The
-// mixed form needs flux; q receives its fragile pairs (cap >= 1).
+// mixed form needs flux; q receives its fragile pairs (cap >= 1), dq the pairs
+// deferred to their own kernel (cap >= 1 with flux; its count zeroed by the caller).
 void force_fp64(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
-                DevStatus *st, void *rec, void *flux, bool all, double *sums, const EventPair *ev, cudaStream_t s);
+                DevStatus *st, void *rec, void *flux, bool all, const RefineQueue &dq, double *sums,
+                const EventPair *ev, cudaStream_t s);
 void force_mixed(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
-                 DevStatus *st, void *rec, void *flux, bool all, const RefineQueue &q, double *sums,
-                 const EventPair *ev, cudaStream_t s);
+                 DevStatus *st, void *rec, void *flux, bool all, const RefineQueue &q, const RefineQueue &dq,
+                 double *sums, const EventPair *ev, cudaStream_t s);
 // The queued pairs of a mixed-form pass evaluated in FP64 from the FP64 mirror
 // (the FP64 form's arithmetic bit for bit), their fluxes stored over the FP32
 // ones at both entries; the queue's count stays on the device.

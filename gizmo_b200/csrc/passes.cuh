@@ -672,17 +672,81 @@ GZ_DEV void push_refine(const RefineQueue &q, bool fragile, long long e, long lo
     }
 }
 
-// Resident 128-thread blocks per multiprocessor the pair kernel asks of the
-// register allocator, each measured at 256^3 against its neighbours. FP32:
-// five (at most 96 registers a thread). FP64: four (at most 128): 96.8 ms
-// against 99.0 at three, 102.8 at two, 101.3 at five.
-template <typename T> constexpr int kForcePairsMinBlocks = sizeof(T) == 4 ? 5 : 4;
+// Resident 128-thread blocks per multiprocessor the pair kernels ask of the
+// register allocator. Every pair once: FP32 five (at most 96 registers; force
+// stage of 2M lognormal / Plummer particles 9.97 / 6.12 ms, at four, six and seven
+// 10.85 / 6.58, 10.08 / 6.11, 10.03 / 6.07), FP64 three (1.41 ms for 110,003
+// lognormal particles, 1.55 at four, 1.74 at five; 7.07, 7.07 and 7.13 ms for a
+// million Plummer particles). Row entries of a subset read both sides' records
+// per lane: FP32 four (1% of 2M: 0.69 ms, 0.74 at five), FP64 three (10% of 1M:
+// 1.61 ms, 1.62 at two, 1.81 at four).
+template <typename T> constexpr int kForcePairsMinBlocks = sizeof(T) == 4 ? 5 : 3;
+template <typename T> constexpr int kForceEntriesMinBlocks = sizeof(T) == 4 ? 4 : 3;
+
+// Pairs that the first attempt at the face does not settle -- the exact Riemann
+// solver, or a retry with other states -- are rare (0.1 to 0.9% of the pairs of
+// clustered and turbulent sets) but were met by 3 to 19% of the warps, which then
+// ran the solver's iteration for one or two lanes. k_force_pairs and
+// k_force_entries therefore only mark such a pair in its flux entries
+// (kDeferred) and queue it, and k_force_deferred evaluates the queued pairs with
+// every lane on one. The same function on the same operands: the fluxes are
+// those of an evaluation in place. Force stage (MFV, FP64, a million Plummer
+// particles) 7.07 against 8.87 ms, 2M Plummer and lognormal particles in the mixed
+// form 6.1 and 10.0 against 7.0 and 11.3 ms, an active tenth of a million in FP64
+// 1.61 against 2.41 ms.
+
+// Row k of a warp's kPairRows rows whose running counts are `incl`: the number
+// of rows whose inclusive count is <= f.
+GZ_DEV int row_of_pair(int incl, int f)
+{
+    int k = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+        const int v = __shfl_sync(0xffffffffu, incl, k + step - 1);
+        if (v <= f) k += step;
+    }
+    return k;
+}
+
+GZ_DEV int warp_inclusive_sum(int v)
+{
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, d);
+        if ((int)(threadIdx.x & 31) >= d) v += u;
+    }
+    return v;
+}
+
+template <typename T> GZ_DEV PairFlux<T> no_flux()
+{
+    PairFlux<T> F;
+    F.valid = 0;
+    F.rho = F.p = T(0);
+    F.v[0] = F.v[1] = F.v[2] = T(0);
+    F.vsig_ts = T(0);
+    return F;
+}
+
+// The pair (lo, hi) of an active-subset pass seen from target t, after its flux:
+// the wake-up test of an inactive neighbour, on the pair's signal speed.
+template <typename T>
+GZ_DEV void entry_wakeup(const Particles &ps, int t, int j, const PairFlux<T> &F, Guard<T> &g, bool &wake)
+{
+    wake = false;
+    if (F.valid && ps.bin_active && !ps.bin_active[ps.timebin[j]]) {
+        const double wake_at = kWakeup * ps.vsig_prev[j];
+        g.near(F.vsig_ts, T(wake_at), F.vsig_ts, 38);
+        wake = (double)F.vsig_ts > wake_at;
+    }
+}
 
 template <typename T>
 __global__ void __launch_bounds__(128, kForcePairsMinBlocks<T>) k_force_pairs(PassParams p, Particles ps, int n_rows,
                                                                               Csr rows, DevStatus *st,
                                                                               const ForceRec<T> *__restrict__ rec,
-                                                                              PairFlux<T> *flux, RefineQueue q)
+                                                                              PairFlux<T> *flux, RefineQueue q,
+                                                                              RefineQueue dq)
 {
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -703,25 +767,14 @@ __global__ void __launch_bounds__(128, kForcePairsMinBlocks<T>) k_force_pairs(Pa
         split = a;
         cnt = (int)(end - a);
     }
-    int incl = cnt;  // inclusive scan of the counts over the warp
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(full, incl, d);
-        if (lane >= d) incl += v;
-    }
+    const int incl = warp_inclusive_sum(cnt);
     const int total = __shfl_sync(full, incl, 31);
     const int mfv = p.method == 1;
     const GConst<T> gc = make_gconst<T>(p.gamma, mfv);
     int stop = 0, stop_index = -1;
     for (int base = 0; base < total; base += 32) {
         const int f = base + lane;
-        // the row of pair f: the number of rows whose inclusive count is <= f
-        int k = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
-            const int v = __shfl_sync(full, incl, k + step - 1);
-            if (v <= f) k += step;
-        }
+        const int k = row_of_pair(incl, f);
         const int excl_k = __shfl_sync(full, incl - cnt, k);
         const long long split_k = __shfl_sync(full, split, k);
         if (f >= total) continue;
@@ -731,20 +784,17 @@ __global__ void __launch_bounds__(128, kForcePairsMinBlocks<T>) k_force_pairs(Pa
         const ForceRec<T> *rip = rec + i;  // shared by the lanes of the row: cached
         const ForceRec<T> rj = ldg_record(rec + j);
         const ForceRec<T> *rjp = &rj;
-        PairFlux<T> F;
-        F.valid = 0;
-        F.rho = F.p = T(0);
-        F.v[0] = F.v[1] = F.v[2] = T(0);
-        F.vsig_ts = T(0);
+        PairFlux<T> F = no_flux<T>();
         Guard<T> g;
         if (rip->m > 0 && rip->rho > 0 && rjp->m > 0 && rjp->rho > 0) {
             double dx, dy, dz;
             const double r2 = sep2(rip->x, rip->y, rip->z, rjp->x, rjp->y, rjp->z, p.box, p.half, dx, dy, dz);
             const T dp[3] = {T(dx), T(dy), T(dz)};
             int pstop = 0;
-            force_pair(p.kernel, mfv, p.selfgravity_off, gc, rip->s, rjp->s, dp, r2, rip->h, rjp->h, F, pstop, g);
-            // a fragile pair's flux (and stop code) comes from its FP64 evaluation, queued below
-            if (g.fragile()) pstop = 0;
+            force_pair<true>(p.kernel, mfv, p.selfgravity_off, gc, rip->s, rjp->s, dp, r2, rip->h, rjp->h, F, pstop, g);
+            // a fragile pair's flux (and stop code) comes from its FP64 evaluation, queued below;
+            // a deferred pair's from k_force_deferred
+            if (g.fragile() || F.valid == kDeferred) pstop = 0;
             if (pstop && !stop) { stop = pstop; stop_index = i; }
         }
         flux[e] = F;
@@ -760,7 +810,9 @@ __global__ void __launch_bounds__(128, kForcePairsMinBlocks<T>) k_force_pairs(Pa
             continue;
         }
         flux[a] = F;
-        push_refine(q, g.fragile(), e, a, i, j, -1);
+        const bool deferred = F.valid == kDeferred;
+        push_refine(dq, deferred, e, a, i, j, -1);
+        push_refine(q, g.fragile() && !deferred, e, a, i, j, -1);
     }
     if (stop) record_status(st, stop, stop_index);
 }
@@ -773,10 +825,12 @@ __global__ void __launch_bounds__(128, kForcePairsMinBlocks<T>) k_force_pairs(Pa
 // goes to k_force<kGather> like the pairs of a pass over every particle. The
 // wake-up test of an inactive neighbour (hydro_functions.h:534-544) runs here.
 template <typename T>
-__global__ void __launch_bounds__(128) k_force_entries(PassParams p, Particles ps, const int *__restrict__ targets,
-                                                       int n_rows, Csr rows, DevStatus *st,
-                                                       const ForceRec<T> *__restrict__ rec, PairFlux<T> *flux,
-                                                       RefineQueue q)
+__global__ void __launch_bounds__(128, kForceEntriesMinBlocks<T>) k_force_entries(PassParams p, Particles ps,
+                                                                                const int *__restrict__ targets,
+                                                                                int n_rows, Csr rows, DevStatus *st,
+                                                                                const ForceRec<T> *__restrict__ rec,
+                                                                                PairFlux<T> *flux, RefineQueue q,
+                                                                                RefineQueue dq)
 {
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -789,24 +843,14 @@ __global__ void __launch_bounds__(128) k_force_entries(PassParams p, Particles p
         first = rows.off[r0 + lane];
         cnt = (int)(rows.off[r0 + lane + 1] - first);
     }
-    int incl = cnt;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(full, incl, d);
-        if (lane >= d) incl += v;
-    }
+    const int incl = warp_inclusive_sum(cnt);
     const int total = __shfl_sync(full, incl, 31);
     const int mfv = p.method == 1;
     const GConst<T> gc = make_gconst<T>(p.gamma, mfv);
     int stop = 0, stop_index = -1;
     for (int base = 0; base < total; base += 32) {
         const int f = base + lane;
-        int k = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
-            const int v = __shfl_sync(full, incl, k + step - 1);
-            if (v <= f) k += step;
-        }
+        const int k = row_of_pair(incl, f);
         const int excl_k = __shfl_sync(full, incl - cnt, k);
         const long long first_k = __shfl_sync(full, first, k);
         if (f >= total) continue;
@@ -815,31 +859,88 @@ __global__ void __launch_bounds__(128) k_force_entries(PassParams p, Particles p
         const int j = rows.nbr[e];
         const int lo = t < j ? t : j, hi = t < j ? j : t;
         const ForceRec<T> rl = ldg_record(rec + lo), rh = ldg_record(rec + hi);
-        PairFlux<T> F;
-        F.valid = 0;
-        F.rho = F.p = T(0);
-        F.v[0] = F.v[1] = F.v[2] = T(0);
-        F.vsig_ts = T(0);
+        PairFlux<T> F = no_flux<T>();
         Guard<T> g;
         if (rl.m > 0 && rl.rho > 0 && rh.m > 0 && rh.rho > 0) {
             double dx, dy, dz;
             const double r2 = sep2(rl.x, rl.y, rl.z, rh.x, rh.y, rh.z, p.box, p.half, dx, dy, dz);
             const T dp[3] = {T(dx), T(dy), T(dz)};
             int pstop = 0;
-            force_pair(p.kernel, mfv, p.selfgravity_off, gc, rl.s, rh.s, dp, r2, rl.h, rh.h, F, pstop, g);
-            // the wake-up test of an inactive neighbour, on the pair's signal speed
-            const bool wake_test = F.valid && ps.bin_active && !ps.bin_active[ps.timebin[j]];
-            const double wake_at = wake_test ? kWakeup * ps.vsig_prev[j] : 0.0;
-            if (wake_test) g.near(F.vsig_ts, T(wake_at), F.vsig_ts, 38);
-            if (g.fragile()) pstop = 0;
-            else if (wake_test && (double)F.vsig_ts > wake_at) atomicMax(ps.wakeup + j, ps.timebin[t] + 1);
-            if (pstop && !stop) { stop = pstop; stop_index = t; }
+            force_pair<true>(p.kernel, mfv, p.selfgravity_off, gc, rl.s, rh.s, dp, r2, rl.h, rh.h, F, pstop, g);
+            if (F.valid != kDeferred) {
+                bool wake;
+                entry_wakeup(ps, t, j, F, g, wake);
+                if (g.fragile()) pstop = 0;
+                else if (wake) atomicMax(ps.wakeup + j, ps.timebin[t] + 1);
+                if (pstop && !stop) { stop = pstop; stop_index = t; }
+            }
         }
         flux[e] = F;
-        push_refine(q, g.fragile(), e, -1, lo, hi, t);
+        const bool deferred = F.valid == kDeferred;
+        push_refine(dq, deferred, e, -1, lo, hi, t);
+        push_refine(q, g.fragile() && !deferred, e, -1, lo, hi, t);
     }
     if (stop) record_status(st, stop, stop_index);
 }
+
+// One deferred pair, evaluated in full: (lo, hi) in canonical orientation, stored
+// at entry e and, when given, at its mirror a.
+template <typename T>
+GZ_DEV void deferred_pair(const PassParams &p, const Particles &ps, const GConst<T> &gc,
+                          const ForceRec<T> *__restrict__ rec, PairFlux<T> *flux, const RefineItem &it, DevStatus *st,
+                          const RefineQueue &q)
+{
+    const ForceRec<T> rl = ldg_record(rec + it.i), rh = ldg_record(rec + it.j);
+    double dx, dy, dz;
+    const double r2 = sep2(rl.x, rl.y, rl.z, rh.x, rh.y, rh.z, p.box, p.half, dx, dy, dz);
+    const T dp[3] = {T(dx), T(dy), T(dz)};
+    int stop = 0;
+    PairFlux<T> F;
+    Guard<T> g;
+    force_pair(p.kernel, gc.mfv, p.selfgravity_off, gc, rl.s, rh.s, dp, r2, rl.h, rh.h, F, stop, g);
+    bool wake = false;
+    const int j = it.t == it.i ? it.j : it.i;
+    if (it.t >= 0) entry_wakeup(ps, it.t, j, F, g, wake);
+    if (!g.fragile()) {
+        if (wake) atomicMax(ps.wakeup + j, ps.timebin[it.t] + 1);
+        if (stop) record_status(st, stop, it.t >= 0 ? it.t : it.i);
+    }
+    flux[it.e] = F;
+    if (it.a >= 0) flux[it.a] = F;
+    push_refine(q, g.fragile(), it.e, it.a, it.i, it.j, it.t);
+}
+
+// The deferred pairs, one per thread over the count the pair kernel left on the
+// device. When more were deferred than the queue holds, the rows are scanned for
+// the marked entries instead and each is evaluated for itself (`all`: every
+// particle a target, no wake-up test).
+template <typename T>
+__global__ void __launch_bounds__(128) k_force_deferred(PassParams p, Particles ps, const int *__restrict__ targets,
+                                                        int n_rows, Csr rows, DevStatus *st,
+                                                        const ForceRec<T> *__restrict__ rec, PairFlux<T> *flux, int all,
+                                                        RefineQueue q, RefineQueue dq)
+{
+    const long long n = (long long)*dq.count;
+    const GConst<T> gc = make_gconst<T>(p.gamma, p.method == 1);
+    const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    if (n <= dq.cap) {
+        for (long long k = first; k < n; k += stride) deferred_pair(p, ps, gc, rec, flux, dq.item[k], st, q);
+        return;
+    }
+    for (long long s = first; s < n_rows; s += stride) {
+        const int t = targets[s];
+        const long long b1 = rows.off[s + 1];
+        for (long long e = rows.off[s]; e < b1; e++) {
+            if (flux[e].valid != kDeferred) continue;
+            const int j = rows.nbr[e];
+            const RefineItem it{e, -1, t < j ? t : j, t < j ? j : t, all ? -1 : t, 0};
+            deferred_pair(p, ps, gc, rec, flux, it, st, q);
+        }
+    }
+}
+
+constexpr unsigned kDeferredBlocks = 148 * 4;
 
 template <typename T, int MODE>
 void launch_force_mode(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
@@ -866,8 +967,8 @@ void launch_force_mode(const PassParams &p, const Particles &ps, const int *targ
 // `sums`: kRowSums x n doubles of scratch.
 template <typename T>
 void launch_force(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
-                  DevStatus *st, void *recbuf, void *fluxbuf, bool all, const RefineQueue &q, double *sums,
-                  const EventPair *ev, cudaStream_t s)
+                  DevStatus *st, void *recbuf, void *fluxbuf, bool all, const RefineQueue &q, const RefineQueue &dq,
+                  double *sums, const EventPair *ev, cudaStream_t s)
 {
     if (n_targets <= 0) return;
     // the record scratch holds the force records, then the gather records
@@ -879,10 +980,12 @@ void launch_force(const PassParams &p, const Particles &ps, const int *targets, 
         PairFlux<T> *flux = (PairFlux<T> *)fluxbuf;
         const long long warps = (n_targets + kPairRows - 1) / kPairRows;
         if (ev) cudaEventRecord(ev->start, s);
-        if (all) k_force_pairs<T><<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(p, ps, n_targets, rows, st, rec, flux, q);
-        else k_force_entries<T><<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(p, ps, targets, n_targets, rows, st, rec,
-                                                                            flux, q);
+        const unsigned blocks = (unsigned)((warps + 3) / 4);
+        if (all) k_force_pairs<T><<<blocks, 128, 0, s>>>(p, ps, n_targets, rows, st, rec, flux, q, dq);
+        else k_force_entries<T><<<blocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, st, rec, flux, q, dq);
         if (ev) cudaEventRecord(ev->stop, s);
+        k_force_deferred<T><<<kDeferredBlocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, st, rec, flux, all ? 1 : 0,
+                                                            q, dq);
         if constexpr (sizeof(T) == sizeof(float)) force_refine(p, ps, q, flux, st, s);
         // one thread per row: the gather's per-entry work is short, and lanes
         // sharing a row would spend more on the cross-lane reduction and on

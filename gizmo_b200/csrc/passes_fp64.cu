@@ -51,10 +51,11 @@ void gradients_fp64(const PassParams &p, const Particles &ps, const int *targets
 }
 
 void force_fp64(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
-                DevStatus *st, void *rec, void *flux, bool all, double *sums, const EventPair *ev, cudaStream_t s)
+                DevStatus *st, void *rec, void *flux, bool all, const RefineQueue &dq, double *sums,
+                const EventPair *ev, cudaStream_t s)
 {
     const RefineQueue none{nullptr, nullptr, 0};
-    launch_force<double>(p, ps, targets, n_targets, rows, tpt, st, rec, flux, all, none, sums, ev, s);
+    launch_force<double>(p, ps, targets, n_targets, rows, tpt, st, rec, flux, all, none, dq, sums, ev, s);
 }
 
 // force_refine: one thread per queued pair, grid-stride over the count the

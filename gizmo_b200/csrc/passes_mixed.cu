@@ -20,10 +20,10 @@ void density_sums_mixed(const PassParams &p, const Particles &ps, const DensityW
 }
 
 void force_mixed(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
-                 DevStatus *st, void *rec, void *flux, bool all, const RefineQueue &q, double *sums,
-                 const EventPair *ev, cudaStream_t s)
+                 DevStatus *st, void *rec, void *flux, bool all, const RefineQueue &q, const RefineQueue &dq,
+                 double *sums, const EventPair *ev, cudaStream_t s)
 {
-    launch_force<float>(p, ps, targets, n_targets, rows, tpt, st, rec, flux, all, q, sums, ev, s);
+    launch_force<float>(p, ps, targets, n_targets, rows, tpt, st, rec, flux, all, q, dq, sums, ev, s);
 }
 
 }  // namespace gz

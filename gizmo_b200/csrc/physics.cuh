@@ -752,10 +752,9 @@ template <typename T> GZ_HD void face_to_flux(ROut<T> &o, const T *n, const GCon
     for (int k = 0; k < 3; k++) o.F.v[k] = v[k] * o.F.rho + n[k] * P;
 }
 
-// Riemann_solver_exact (reimann.h:625-664). Taken on a small fraction of
-// faces only, but inlined: called out of line, the solver's inputs and
-// outputs had to be addressable in local memory around the call, and the
-// pair kernels ran 5% (FP32) and 4% (FP64) slower at 256^3.
+// Riemann_solver_exact (reimann.h:625-664). Inlined: called out of line, the
+// solver's inputs and outputs had to be addressable in local memory around the
+// call, and the kernels that hold it ran 4-5% slower.
 template <typename T>
 __host__ __device__ __forceinline__ void riemann_exact(const RVec<T> &rv, ROut<T> &o, const T *n, T vL, T vR, T cL, T cR,
                                                     const GConst<T> &gc, int &stop, Guard<T> &g)
@@ -780,11 +779,12 @@ __host__ __device__ __forceinline__ void riemann_exact(const RVec<T> &rv, ROut<T
     if (gc.mfv) face_to_flux(o, n, gc);
 }
 
-// Riemann_solver, hydro branch (reimann.h:282-370); rv taken by value as in the reference
-template <typename T>
-GZ_HD void riemann_solver(RVec<T> rv, ROut<T> &o, const T *n, T ptl, const GConst<T> &gc, int &stop, Guard<T> &g)
+// Riemann_solver, hydro branch (reimann.h:282-370); rv taken by value as in the reference.
+// With DEFER a face that needs the exact solver is not solved: true is returned.
+template <bool DEFER, typename T>
+GZ_HD bool riemann_solver(RVec<T> rv, ROut<T> &o, const T *n, T ptl, const GConst<T> &gc, int &stop, Guard<T> &g)
 {
-    if ((rv.L.p < T(0) && rv.R.p < T(0)) || (rv.L.rho < T(0)) || (rv.R.rho < T(0))) { o.P_M = T(0); return; }
+    if ((rv.L.p < T(0) && rv.R.p < T(0)) || (rv.L.rho < T(0)) || (rv.R.rho < T(0))) { o.P_M = T(0); return false; }
     rv.L.cs = Real<T>::sqrt_(gc.G0 * rv.L.p / rv.L.rho);
     rv.R.cs = Real<T>::sqrt_(gc.G0 * rv.R.p / rv.R.rho);
     rv.L.u = rv.L.p / (gc.G9 * rv.L.rho);
@@ -807,7 +807,11 @@ GZ_HD void riemann_solver(RVec<T> rv, ROut<T> &o, const T *n, T ptl, const GCons
         riemann_kt(rv, o, n, vL, vR, cL, cR, hL, hR, gc);
     }
     g.near(o.P_M, ptl, ptl, 21);
-    if ((o.P_M < T(0)) || Real<T>::isnan_(o.P_M) || (o.P_M > ptl)) riemann_exact(rv, o, n, vL, vR, cL, cR, gc, stop, g);
+    if ((o.P_M < T(0)) || Real<T>::isnan_(o.P_M) || (o.P_M > ptl)) {
+        if constexpr (DEFER) return true;
+        riemann_exact(rv, o, n, vL, vR, cL, cR, gc, stop, g);
+    }
+    return false;
 }
 
 // reconstruct_face_states, non-MHD (reimann.h:125-244).
@@ -897,8 +901,9 @@ template <typename T> struct Side {
 template <typename T> struct __align__(16) PairFlux {
     T rho, p, v[3];  // Fluxes.{rho,p,v} after face-area scaling and the MFM switch
     T vsig_ts;       // vsig + |c_i - c_j|, for MaxSignalVel
-    int valid;       // inside support (r < max(h_i,h_j), r > 0, j has mass/density)
+    int valid;       // inside support (r < max(h_i,h_j), r > 0, j has mass/density); kDeferred: not evaluated yet
 };
+constexpr int kDeferred = 2;
 
 // hydro_accumulate_neighbor (hydro_functions.h:56-546) pair part: kernels at
 // h_i and h_j, signal speed, then the meshless core
@@ -909,7 +914,10 @@ template <typename T> struct __align__(16) PairFlux {
 // `g` collects the pair's fragile decisions (Guard<float>: a mixed-form pair
 // whose branch may differ from the FP64 form's, or whose arithmetic cancels
 // beyond FP32's reach; the caller evaluates it again in FP64).
-template <typename T>
+// With DEFER a pair whose first attempt does not settle the face (the exact
+// solver, or a retry) is left: out.valid is kDeferred, out and g mean nothing
+// else, and the caller has it evaluated without DEFER elsewhere.
+template <bool DEFER = false, typename T>
 GZ_HD void force_pair(int kf, int mfv, int selfgravity_off, const GConst<T> &gc, const Side<T> &I, const Side<T> &J,
                        const T dp[3], double r2d, double hi_d, double hj_d, PairFlux<T> &out, int &stop, Guard<T> &g)
 {
@@ -1040,7 +1048,8 @@ GZ_HD void force_pair(int kf, int mfv, int selfgravity_off, const GConst<T> &gc,
                 }
                 lim = attempt == 1 ? T(1.4) * ptl : T(2.0) * ptl;
             }
-            riemann_solver(rv, ro, n, lim, gc, stop, g);
+            const bool unsolved = riemann_solver<DEFER>(rv, ro, n, lim, gc, stop, g);
+            if (DEFER && unsolved) { out.valid = kDeferred; return; }
             bool retry = (ro.P_M < T(0)) || Real<T>::isnan_(ro.P_M);
             if (attempt == 0) {
                 g.near(ro.P_M, T(1.4) * ptl, ptl, 27);
@@ -1048,6 +1057,7 @@ GZ_HD void force_pair(int kf, int mfv, int selfgravity_off, const GConst<T> &gc,
             }
             if (Real<T>::isnan_(ro.P_M)) g.flag(28);  // a NaN star pressure: decided in FP64
             if (!retry) break;
+            if constexpr (DEFER) { out.valid = kDeferred; return; }
             if (attempt == 2) stop = 1234;
         }
         if (!((ro.P_M > T(0)) && (!Real<T>::isnan_(ro.P_M)))) { Fl = Crv<T>{}; break; }

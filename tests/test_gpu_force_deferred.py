@@ -1,0 +1,66 @@
+"""Force pairs that the first attempt at the face does not settle (the exact Riemann solver, the retries) are
+marked and evaluated by a kernel of their own, from a queue, or, when more are deferred than the queue holds,
+from the marked row entries. Against the oracle (the parity tolerances) on sets of which most faces are
+deferred, in every pass that has the two routes: every particle and an active subset, plain and captured; and
+the queue's two routes against each other bit for bit."""
+import numpy as np
+import pytest
+
+from gizmo_b200 import abi, ics
+from gizmo_b200.hydro import HydroPass
+from oracle import oracle as O
+from tests._util import field_err, riemann_fallback_case
+
+pytestmark = pytest.mark.gpu
+FORCE = ("accel", "dudt", "vsig", "dtmass", "dmass", "gravwork")
+
+
+@pytest.mark.parametrize("method", [abi.METHOD_MFM, abi.METHOD_MFV], ids=["mfm", "mfv"])
+@pytest.mark.parametrize("mach", [5.0, 50.0])
+def test_deferred_faces_match_the_oracle(method, mach):
+    wl = riemann_fallback_case(method, mach=mach)
+    wl.params.precision = abi.PRECISION_FP64
+    with HydroPass(wl.params) as hp:
+        hp.upload_workload(wl)
+        hp.full_pass()
+        g = hp.download()
+        hp.restage()
+        hp.hydro_pass(graph=True)
+        again = hp.download()
+        assert hp.graph_stats()["fallbacks"] == 0
+    for k in g:
+        assert np.array_equal(g[k], again[k]), k
+    st = O.new_state(wl.n, wl.inputs())
+    orc = O.Oracle(wl.params, "port")
+    assert orc.density(st) == 0
+    for k in ("h", "num_ngb", "drkern", "divvel", "rho", "pressure", "nvt", "cond", "fce", "pvel", "grad_rho", "grad_p",
+              "grad_v"):
+        st[k][...] = g[k].reshape(st[k].shape)
+    assert orc.force(st) == 0
+    for k in FORCE:
+        assert field_err(k, g[k], st[k].reshape(g[k].shape), 1e-3) < 1e-10, k
+
+
+@pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_MIXED], ids=["fp64", "mixed"])
+def test_more_deferred_pairs_than_the_queue_holds(precision):
+    """48^3 cells at Mach 200: over 65,536 deferred pairs, so a pass scans its marked entries; the same cells as an
+    active list of all but one (the row entries' route), and a slice of them small enough for the queue."""
+    wl = riemann_fallback_case(abi.METHOD_MFM, n1=48, mach=200.0)
+    wl.params.precision = precision
+    part = np.arange(0, 2000, dtype=np.int32)
+    # (an active list whose fragile pairs outgrow the mixed form's queue is refused, so only FP64 takes the long one)
+    most = np.arange(wl.n - 1 if precision == abi.PRECISION_FP64 else 1500, dtype=np.int32)
+    with HydroPass(wl.params) as hp:
+        hp.upload_workload(wl)
+        hp.density()
+        hp.hydro_gradient_calc()
+        hp.hydro_force()
+        full = hp.download(list(FORCE))
+        hp.hydro_force(part)
+        small = hp.download(list(FORCE))
+        hp.hydro_force(most)
+        large = hp.download(list(FORCE))
+    assert np.isfinite(full["accel"]).all()
+    for k in ("accel", "dudt", "vsig"):  # the same terms, summed in the rows' order in each
+        assert np.array_equal(full[k][part], small[k][part]), k
+        assert np.array_equal(full[k][most], large[k][most]), k
