@@ -857,6 +857,57 @@ int sym_rows_from_density(gz_context *c)
     return 0;
 }
 
+// Symmetric rows of a target list in one walk (the count walk, scan and fill walk
+// of build_rows visit every candidate twice: 1.68 against 1.02 ms for the gradient
+// stage of 1% of 2M particles, 4.62 against 2.70 for 10% of 1M): cap slots per target in scratch
+// (the walk counts every row in full), their counts scanned into offsets, the
+// rows copied to their places, and the few longer than cap filled by a walk of
+// their own. `fits` is false when there is no room for the slots: nothing is
+// built then.
+int sym_rows_one_walk(gz_context *c, int rows, long long *total, bool *fits)
+{
+    cudaStream_t s = c->stream;
+    const int cap = 32 * (int)std::ceil(c->row_slots * c->prm.des_num_ngb / 32.0);
+    const long long slots = (long long)rows * cap;
+    *fits = slots <= (long long)INT32_MAX && try_ensure(c->s_tmp, sizeof(int) * (size_t)slots);
+    if (!*fits) return 0;
+    const size_t R = (size_t)rows;
+    if (ensure(c, c->s_counts, sizeof(long long) * R) || ensure(c, c->s_off, sizeof(long long) * (R + 1)) ||
+        ensure(c, c->work, sizeof(int)) || ensure(c, c->pad_list, sizeof(int) * R) ||
+        ensure(c, c->pad_counts, sizeof(long long) * R) || ensure(c, c->n_sel, sizeof(int) * 2))
+        return c->err;
+    Tree t = tree_view(c);
+    const int *targets = ptr<int>(c->targets);
+    long long *counts = ptr<long long>(c->s_counts), *off = ptr<long long>(c->s_off);
+    walk_timed(c, t, ptr<double>(c->x), ptr<double>(c->y), ptr<double>(c->z), ptr<double>(c->h), ptr<double>(c->h), 1,
+               targets, rows, counts, nullptr, ptr<int>(c->s_tmp), cap, ptr<DevStatus>(c->status), ptr<int>(c->work), s);
+    GZ_CUDA(c, cudaGetLastError());
+    GZ_CUDA(c, cudaMemsetAsync(off, 0, sizeof(long long), s));
+    size_t tmp = 0;
+    cub::DeviceScan::InclusiveSum(nullptr, tmp, counts, off + 1, rows, s);
+    if (ensure(c, c->cub_tmp, tmp)) return c->err;
+    cub::DeviceScan::InclusiveSum(c->cub_tmp.p, tmp, counts, off + 1, rows, s);
+    GZ_CUDA(c, cudaMemsetAsync(c->n_sel.p, 0, sizeof(int), s));
+    long_rows(rows, targets, counts, off, cap, ptr<int>(c->pad_list), ptr<long long>(c->pad_counts), ptr<int>(c->n_sel), s);
+    int n_long = 0;
+    GZ_CUDA(c, cudaMemcpyAsync(total, off + rows, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    GZ_CUDA(c, cudaMemcpyAsync(&n_long, c->n_sel.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    GZ_CUDA(c, cudaStreamSynchronize(s));
+    c->launches += 2;
+    if (*total > (long long)INT32_MAX * 4) return fail(c, GZ_ERR_CAPACITY, "neighbour rows exceed capacity");
+    if (grow_keep(c, c->s_nbr, c->s_nbr_cap, 0, *total)) return c->err;
+    copy_rows(rows, counts, off, cap, ptr<int>(c->s_tmp), ptr<int>(c->s_nbr), s);
+    c->launches++;
+    if (n_long > 0) {
+        walk_timed(c, t, ptr<double>(c->x), ptr<double>(c->y), ptr<double>(c->z), ptr<double>(c->h), ptr<double>(c->h), 1,
+                   ptr<int>(c->pad_list), n_long, nullptr, ptr<long long>(c->pad_counts), ptr<int>(c->s_nbr), 0,
+                   ptr<DevStatus>(c->status), ptr<int>(c->work), s);
+        c->launches++;
+    }
+    GZ_CUDA(c, cudaGetLastError());
+    return 0;
+}
+
 int build_sym_rows(gz_context *c, int rows, bool all)
 {
     if (all && c->dens_all && rows == c->n && c->n > 0) {
@@ -864,8 +915,10 @@ int build_sym_rows(gz_context *c, int rows, bool all)
     } else {
         if (refresh_hmax(c)) return c->err;
         long long total = 0;
-        if (build_rows(c, ptr<double>(c->h), 1, ptr<int>(c->targets), rows, c->s_counts, c->s_off, c->s_nbr,
-                       c->s_nbr_cap, &total))
+        bool fits = false;
+        if (sym_rows_one_walk(c, rows, &total, &fits)) return c->err;
+        if (!fits && build_rows(c, ptr<double>(c->h), 1, ptr<int>(c->targets), rows, c->s_counts, c->s_off, c->s_nbr,
+                                c->s_nbr_cap, &total))
             return c->err;
         c->pairs_symmetric = total;
     }
@@ -982,8 +1035,7 @@ __global__ void k_g_prep(GraphState *gs, int cap0, int cap1, long long nbr_cap, 
         g.need = g.base + (long long)g.n_grow * g.cap;
         if (g.need > nbr_cap) g.fail |= kGraphFailRows;
         // the walk mode of walk_rows (both modes write the same rows)
-        const bool sparse = (long long)g.n_grow * 4 < n_particles;
-        g.walk_solo = (g.n_grow == 1 || (sparse && (g.n_grow + 31) / 32 < group_warps)) ? 1 : 0;
+        g.walk_solo = walk_one_target_per_warp(g.n_grow, n_particles, group_warps, false) ? 1 : 0;
     }
 }
 
@@ -1192,6 +1244,12 @@ int density_caps(const gz_context *c, int *cap0, int *cap1)
 // (no error recorded) when the device has no room for them: the pass then
 // runs plain.
 constexpr int kNoRoom = -1;
+
+// queue room for the deferred force pairs of `entries` symmetric row entries:
+// one pair in 16 (under 1 in 100 is deferred on the sets measured; when more
+// are, k_force_deferred scans the rows instead)
+long long deferred_cap(long long entries) { return std::max(65536ll, entries / 32); }
+
 int graph_buffers(gz_context *c, long long *sym_cap, long long *rq_cap, bool with_restage)
 {
     const int n = c->n;
@@ -1420,6 +1478,9 @@ int capture_gradients_force(gz_context *c, cudaStream_t s, long long rq_cap)
     gradients_fp64(c->pp, ps, ptr<int>(c->targets), n, rows, lanes_per_row(c, n, 1), c->rec.p, nullptr, s);
     if (c->have_bins) GZ_CUDA(c, cudaMemsetAsync(c->wakeup.p, 0, sizeof(int) * N, s));
     force_preloop(c->pp, ps, ptr<int>(c->targets), n, s);
+    GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), s));
+    const RefineQueue dq{ptr<RefineItem>(c->dq), ptr<unsigned long long>(c->deferred),
+                         (long long)(c->dq.bytes / sizeof(RefineItem))};
     if (c->prm.precision == GZ_PRECISION_MIXED) {
         GZ_CUDA(c, cudaMemsetAsync(c->refined.p, 0, sizeof(unsigned long long), s));
         const RefineQueue q{ptr<RefineItem>(c->rq), ptr<unsigned long long>(c->refined), rq_cap};
@@ -2082,6 +2143,15 @@ int gz_hydro_force(gz_context *c, const int *active, int n_active)
                 return c->err;
             GZ_CUDA(c, cudaMemsetAsync(c->refined.p, 0, sizeof(unsigned long long), c->stream));
             q = RefineQueue{ptr<RefineItem>(c->rq), ptr<unsigned long long>(c->refined), cap};
+        }
+        RefineQueue dq{nullptr, nullptr, 0};
+        if (flux) {
+            if (ensure(c, c->deferred, sizeof(unsigned long long)) ||
+                ensure(c, c->dq, sizeof(RefineItem) * (size_t)deferred_cap(c->pairs_symmetric)))
+                return c->err;
+            GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), c->stream));
+            dq = RefineQueue{ptr<RefineItem>(c->dq), ptr<unsigned long long>(c->deferred),
+                             (long long)(c->dq.bytes / sizeof(RefineItem))};
         }
         // the rows' sums before the writeback go to the density accumulators
         // (17 x n doubles, unused between density passes)

@@ -770,6 +770,44 @@ __global__ void k_padded_rows(int na, const int *__restrict__ t, const long long
     }
 }
 
+// The rows of a padded fill longer than their cap slots: their targets and exact
+// offsets (in any order: a row's content does not depend on it).
+__global__ void k_long_rows(int rows, const int *__restrict__ t, const long long *__restrict__ counts,
+                            const long long *__restrict__ off, int cap, int *list, long long *list_off, int *n)
+{
+    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a >= rows || counts[a] <= cap) return;
+    const int k = atomicAdd(n, 1);
+    list[k] = t[a];
+    list_off[k] = off[a];
+}
+
+// The rows that fit their slots copied to their offsets, eight lanes a row.
+__global__ void __launch_bounds__(256) k_copy_rows(int rows, const long long *__restrict__ counts,
+                                                   const long long *__restrict__ off, int cap,
+                                                   const int *__restrict__ padded, int *nbr)
+{
+    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long a = g >> 3;
+    if (a >= rows) return;
+    const long long c = counts[a], o = off[a];
+    if (c > cap) return;
+    for (int k = (int)(g & 7); k < c; k += 8) nbr[o + k] = padded[a * cap + k];
+}
+
+void long_rows(int rows, const int *t, const long long *counts, const long long *off, int cap, int *list,
+               long long *list_off, int *n, cudaStream_t s)
+{
+    if (rows > 0) k_long_rows<<<(rows + 255) / 256, 256, 0, s>>>(rows, t, counts, off, cap, list, list_off, n);
+}
+
+void copy_rows(int rows, const long long *counts, const long long *off, int cap, const int *padded, int *nbr,
+               cudaStream_t s)
+{
+    if (rows > 0)
+        k_copy_rows<<<(unsigned)(((long long)rows * 8 + 255) / 256), 256, 0, s>>>(rows, counts, off, cap, padded, nbr);
+}
+
 void padded_rows(int na, const int *t, const long long *counts, int cap, long long base, long long *beg,
                  long long *end, unsigned char *over, cudaStream_t s)
 {
@@ -876,9 +914,7 @@ void walk_rows(const Tree &t, const double *x, const double *y, const double *z,
     // list (the rows rebuilt after an h regrowth, scattered through the box)
     // gets one warp per target instead: as groups it would run on a few
     // warps, each walking 32 unrelated regions one after another.
-    const long long group_warps = walk_group_warps();
-    const bool sparse = (long long)n_targets * 4 < (long long)t.n_particles;
-    const bool solo = n_targets == 1 || (sparse && (n_targets + 31) / 32 < group_warps);
+    const bool solo = walk_one_target_per_warp(n_targets, t.n_particles, walk_group_warps(), symmetric);
 #define GZ_WALK(S, F, O) launch_walk<S, F, O>(t, x, y, z, reach, hsym, targets, n_targets, counts, off, nbr, cap, st, next_group, s)
     if (symmetric) {
         if (solo) { if (nbr) GZ_WALK(true, true, true); else GZ_WALK(true, false, true); }

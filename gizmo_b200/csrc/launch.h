@@ -37,12 +37,33 @@ void walk_rows_graph(const Tree &t, const double *x, const double *y, const doub
 // warps the group-mode walk holds resident (the walk takes one warp per
 // target when a sparse list's groups would not fill them)
 long long walk_group_warps();
+// The walk's mode for n_targets targets among n_particles. Groups take 32
+// consecutive targets down the tree at once, but a short list of scattered
+// targets gives few groups, each of which walks 32 unrelated regions: one warp per
+// target is faster while the groups would fill less than a quarter of the
+// resident warps (density rows rebuilt after an h regrowth: density stage of a
+// million Plummer particles 16.65 ms, 17.5 when groups had to fill all of them,
+// 17.1 and 18.2 at a 16th and a 64th). Symmetric rows are only walked for
+// active lists, whose targets lie in the same dense regions: a 16th (1% of 2M
+// particles active: gradient stage 0.84 against 1.03 ms at a quarter, 1.02 at
+// all; 10% of 1M: 1.29 ms, 2.70 at all).
+__host__ __device__ inline bool walk_one_target_per_warp(long long n_targets, long long n_particles,
+                                                         long long group_warps, bool symmetric)
+{
+    if (n_targets == 1) return true;
+    return n_targets * 4 < n_particles && (n_targets + 31) / 32 * (symmetric ? 16 : 4) < group_warps;
+}
 void walk_over_graph(const Tree &t, const double *x, const double *y, const double *z, const double *reach,
                      const int *list, const long long *off, GraphState *gs, int *nbr, DevStatus *st, int blocks,
                      cudaStream_t s);
 // rows of a padded fill (cap > 0 above): [beg, end) for the rows that fit, over[a] = 1 for the others
 void padded_rows(int na, const int *t, const long long *counts, int cap, long long base, long long *beg,
                  long long *end, unsigned char *over, cudaStream_t s);
+// the rows of a padded fill longer than their slots (targets and offsets), and the others copied to their offsets
+void long_rows(int rows, const int *t, const long long *counts, const long long *off, int cap, int *list,
+               long long *list_off, int *n, cudaStream_t s);
+void copy_rows(int rows, const long long *counts, const long long *off, int cap, const int *padded, int *nbr,
+               cudaStream_t s);
 
 // symmetric rows derived from the density rows of a pass over all particles
 void sym_split(int n, const double *x, const double *y, const double *z, const double *h, double box,
