@@ -1303,12 +1303,6 @@ int graph_buffers(gz_context *c, long long *sym_cap, long long *rq_cap, bool wit
     *sym_cap = std::min<long long>({sc, (long long)(c->s_nbr.bytes / sizeof(int)), (long long)(c->s_tmp.bytes / sizeof(int)),
                                     (long long)(c->pflux.bytes / pair_flux_bytes(mixed))});
     *rq_cap = rq;
-
-// queue room for the deferred force pairs of `entries` symmetric row entries:
-// one pair in 16 (under 1 in 100 is deferred on the sets measured; when more
-// are, k_force_deferred scans the rows instead)
-long long deferred_cap(long long entries) { return std::max(65536ll, entries / 32); }
-
     return 0;
 }
 
@@ -1533,9 +1527,6 @@ int graph_capture(gz_context *c, long long sym_cap, long long rq_cap, bool with_
             if ((rc = enqueue_restage(c, true))) break;
             k_g_tree_check<<<1, 1, 0, s>>>(ptr<TreeBuild>(c->t_build), ptr<GraphState>(c->gstate));
             restage_kernels = c->launches - l0 + 1 + 2 * 22 + 1 + 1;  // + tree build, bottom-up pass, check
-    GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), s));
-    const RefineQueue dq{ptr<RefineItem>(c->dq), ptr<unsigned long long>(c->deferred),
-                         (long long)(c->dq.bytes / sizeof(RefineItem))};
             if ((rc = check_last(c, "restage"))) break;
         }
         // the inputs a plain pass would restart from
@@ -2205,15 +2196,6 @@ int gz_set_boxes(gz_context *c, int n_boxes, const int64_t *counts)
         c->box_bits = 0;
     } else {
         for (int b = 0; b < n_boxes; b++)
-        RefineQueue dq{nullptr, nullptr, 0};
-        if (flux) {
-            if (ensure(c, c->deferred, sizeof(unsigned long long)) ||
-                ensure(c, c->dq, sizeof(RefineItem) * (size_t)deferred_cap(c->pairs_symmetric)))
-                return c->err;
-            GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), c->stream));
-            dq = RefineQueue{ptr<RefineItem>(c->dq), ptr<unsigned long long>(c->deferred),
-                             (long long)(c->dq.bytes / sizeof(RefineItem))};
-        }
             if (counts[b] < 0) return GZ_ERR_ARG;
         int bits = 0;
         while ((1 << bits) < n_boxes) bits++;
