@@ -652,6 +652,24 @@ __global__ void __launch_bounds__(256) k_force_finish(PassParams p, Particles ps
 // fluxes.
 constexpr int kPairRows = 32;
 
+// Rows per warp of the pair kernels: kPairRows, or fewer (down to 2) when the
+// warps would not fill the resident ones four times over -- a small set otherwise
+// leaves the multiprocessors idle, and a last wave of long-running warps keeps
+// most of them waiting. Force stage at 32 rows a warp and at this rule: 4,096 lattice
+// cells FP64 0.21 / 0.09 ms, 64,000 0.36 / 0.31, 110,003 lognormal particles 1.46 /
+// 1.35, 1% of 2M active (mixed) 0.69 / 0.54, 10% of 1M active (FP64) 1.62 / 1.55;
+// twice and half the warps asked for are within 3% of it.
+inline int pair_rows(long long n_rows, int blocks_per_sm)
+{
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long want = 4ll * sms * blocks_per_sm * 4;  // 128-thread blocks: four warps each
+    int r = kPairRows;
+    while (r > 2 && n_rows < want * r) r /= 2;
+    return r;
+}
+
 // Queues this lane's pair for the FP64 re-evaluation when `fragile`. Called by
 // every lane that reaches it; the lanes that arrive together take one atomic
 // for all of their pushes (the count is one address for the whole launch).
@@ -742,7 +760,7 @@ GZ_DEV void entry_wakeup(const Particles &ps, int t, int j, const PairFlux<T> &F
 }
 
 template <typename T>
-__global__ void __launch_bounds__(128, kForcePairsMinBlocks<T>) k_force_pairs(PassParams p, Particles ps, int n_rows,
+__global__ void __launch_bounds__(128, kForcePairsMinBlocks<T>) k_force_pairs(PassParams p, Particles ps, int n_rows, int rows_per_warp,
                                                                               Csr rows, DevStatus *st,
                                                                               const ForceRec<T> *__restrict__ rec,
                                                                               PairFlux<T> *flux, RefineQueue q,
@@ -750,13 +768,13 @@ __global__ void __launch_bounds__(128, kForcePairsMinBlocks<T>) k_force_pairs(Pa
 {
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    const long long r0 = warp * kPairRows;
+    const long long r0 = warp * rows_per_warp;
     if (r0 >= n_rows) return;  // the whole warp leaves together
     const unsigned full = 0xffffffffu;
     // lane k: row r0 + k, its first entry with j > i and the number of such entries
     long long split = 0;
     int cnt = 0;
-    if (lane < kPairRows && r0 + lane < n_rows) {
+    if (lane < rows_per_warp && r0 + lane < n_rows) {
         const int i = (int)(r0 + lane);
         long long a = rows.off[i], b = rows.off[i + 1];
         const long long end = b;
@@ -827,19 +845,20 @@ __global__ void __launch_bounds__(128, kForcePairsMinBlocks<T>) k_force_pairs(Pa
 template <typename T>
 __global__ void __launch_bounds__(128, kForceEntriesMinBlocks<T>) k_force_entries(PassParams p, Particles ps,
                                                                                 const int *__restrict__ targets,
-                                                                                int n_rows, Csr rows, DevStatus *st,
+                                                                                int n_rows, int rows_per_warp, Csr rows,
+                                                                                DevStatus *st,
                                                                                 const ForceRec<T> *__restrict__ rec,
                                                                                 PairFlux<T> *flux, RefineQueue q,
                                                                                 RefineQueue dq)
 {
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    const long long r0 = warp * kPairRows;
+    const long long r0 = warp * rows_per_warp;
     if (r0 >= n_rows) return;  // the whole warp leaves together
     const unsigned full = 0xffffffffu;
     long long first = 0;
     int cnt = 0;
-    if (lane < kPairRows && r0 + lane < n_rows) {
+    if (lane < rows_per_warp && r0 + lane < n_rows) {
         first = rows.off[r0 + lane];
         cnt = (int)(rows.off[r0 + lane + 1] - first);
     }
@@ -978,11 +997,12 @@ void launch_force(const PassParams &p, const Particles &ps, const int *targets, 
         ps, p.gamma, rec, grec);
     if (fluxbuf) {
         PairFlux<T> *flux = (PairFlux<T> *)fluxbuf;
-        const long long warps = (n_targets + kPairRows - 1) / kPairRows;
+        const int per_warp = pair_rows(n_targets, all ? kForcePairsMinBlocks<T> : kForceEntriesMinBlocks<T>);
+        const long long warps = ((long long)n_targets + per_warp - 1) / per_warp;
         if (ev) cudaEventRecord(ev->start, s);
         const unsigned blocks = (unsigned)((warps + 3) / 4);
-        if (all) k_force_pairs<T><<<blocks, 128, 0, s>>>(p, ps, n_targets, rows, st, rec, flux, q, dq);
-        else k_force_entries<T><<<blocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, st, rec, flux, q, dq);
+        if (all) k_force_pairs<T><<<blocks, 128, 0, s>>>(p, ps, n_targets, per_warp, rows, st, rec, flux, q, dq);
+        else k_force_entries<T><<<blocks, 128, 0, s>>>(p, ps, targets, n_targets, per_warp, rows, st, rec, flux, q, dq);
         if (ev) cudaEventRecord(ev->stop, s);
         k_force_deferred<T><<<kDeferredBlocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, st, rec, flux, all ? 1 : 0,
                                                             q, dq);
