@@ -47,10 +47,11 @@ long long walk_group_warps();
 // active lists, whose targets lie in the same dense regions: a 16th (1% of 2M
 // particles active: gradient stage 0.84 against 1.03 ms at a quarter, 1.02 at
 // all; 10% of 1M: 1.29 ms, 2.70 at all).
+constexpr int kSoloWaves = 4;
 __host__ __device__ inline bool walk_one_target_per_warp(long long n_targets, long long n_particles,
                                                          long long group_warps, bool symmetric)
 {
-    if (n_targets == 1) return true;
+    if (n_targets <= kSoloWaves * group_warps) return true;
     return n_targets * 4 < n_particles && (n_targets + 31) / 32 * (symmetric ? 16 : 4) < group_warps;
 }
 void walk_over_graph(const Tree &t, const double *x, const double *y, const double *z, const double *reach,
