@@ -792,7 +792,7 @@ int build_tree(gz_context *c)
                       ptr<TreeBuild>(c->t_build), (int)cap, c->leaf_max, c->box_bits / 3,
                       c->box_bits ? ptr<int>(c->box_of) : nullptr, c->box_bits ? ptr<int>(c->root_of) : nullptr,
                       c->sms * 8, s);
-    c->launches += 1 + 2 * 22;
+    c->launches += tree_build_launches(n);
     TreeBuild tb{};
     GZ_CUDA(c, cudaMemcpyAsync(&tb, c->t_build.p, sizeof(tb), cudaMemcpyDeviceToHost, s));
     GZ_CUDA(c, cudaStreamSynchronize(s));
@@ -1526,7 +1526,7 @@ int graph_capture(gz_context *c, long long sym_cap, long long rq_cap, bool with_
             const long long l0 = c->launches;
             if ((rc = enqueue_restage(c, true))) break;
             k_g_tree_check<<<1, 1, 0, s>>>(ptr<TreeBuild>(c->t_build), ptr<GraphState>(c->gstate));
-            restage_kernels = c->launches - l0 + 1 + 2 * 22 + 1 + 1;  // + tree build, bottom-up pass, check
+            restage_kernels = c->launches - l0 + tree_build_launches(n) + 1 + 1;  // + tree build, bottom-up pass, check
             if ((rc = check_last(c, "restage"))) break;
         }
         // the inputs a plain pass would restart from

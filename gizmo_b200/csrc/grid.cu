@@ -26,6 +26,8 @@
 //   symmetric r2 > 0 and !(r2 >= h_i^2 and r2 >= h_j^2) (gradients, force)
 #include <cub/cub.cuh>
 
+#include <cooperative_groups.h>
+
 #include <atomic>
 
 #include "launch.h"
@@ -119,67 +121,121 @@ __global__ void k_tree_count(const unsigned long long *__restrict__ keys, int L,
 }
 
 // ---------------------------------------------- the octree built on the device
-// All levels in one stream of launches with no host round trip: each level's
-// nodes take their children's places from a counter (a node's children are
-// contiguous and in octant order; the order of the nodes of a level depends on
-// the atomics, and nothing downstream depends on it: the walks follow child
-// ranges, the boxes are reduced bottom-up). A level that would pass the node
-// capacity sets `fail` and the host builds the tree level by level instead.
-__global__ void k_tree_init(TreeBuild *tb, int4 *node, int *parent, int n)
+// All levels with no host round trip: each level's nodes take their children's
+// places from a counter (a node's children are contiguous and in octant order;
+// the order of the nodes of a level depends on the atomics, and nothing
+// downstream depends on it: the walks follow child ranges, the boxes are reduced
+// bottom-up). A level that would pass the node capacity sets `fail` and the host
+// builds the tree level by level instead.
+//
+// What bounds a level is the latency of the binary searches for the children's
+// bounds, so eight lanes take a node, one bound each (one thread a node, its
+// seven searches one after another: 433 us for the 22 levels of 2M particles).
+// The narrow levels at the top, and whole trees of small sets, are built by one
+// cluster of thread blocks, its barrier between levels, instead of two launches a
+// level; the wide levels get a launch each, whose last block advances the state.
+// Restage of 4,096 / 110,003 / 2M particles 0.20 / 0.33 / 0.94 ms against 0.42 /
+// 0.61 / 1.40 ms with 44 launches of one thread a node and the separate memsets
+// and gathers it also had.
+constexpr int kNodeLanes = 8;
+constexpr int kTopBlocks = 8, kTopThreads = 1024;                  // the cluster: one node per 8 lanes at a time
+constexpr int kTopNodes = kTopBlocks * kTopThreads / kNodeLanes;
+constexpr int kTopLimit = 2 * kTopNodes;                           // a level above this is left to a launch of its own
+
+// One node of level L by its 8 lanes (`lane` of them, on `mask`).
+GZ_DEV void split_node(const unsigned long long *__restrict__ keys, int4 *node, int *parent, TreeBuild *tb, int i,
+                       int L, int end, int cap, int leaf_max, int split_levels, const int *__restrict__ box_of,
+                       int *root_of, int lane, unsigned mask)
 {
-    node[0] = make_int4(0, n, -1, 0);
-    parent[0] = -1;
-    TreeBuild t{};
-    t.level_cnt = n > 0 ? 1 : 0;
-    t.total = t.level_cnt;
-    *tb = t;
+    const int4 nd = __ldcg(node + i);
+    if (lane == 0 && box_of && L == split_levels) root_of[box_of[nd.x]] = i;  // one node per box
+    if (!((nd.y > leaf_max || L < split_levels) && L < kBits)) return;        // a leaf, as it was written
+    const int a = nd.x, b = nd.x + nd.y;
+    const int shift = 3 * (kBits - L - 1);
+    const unsigned long long prefix = keys[a] >> (shift + 3);
+    const int lo = lane == 0 ? a : lower_bound_key(keys, a, b, ((prefix << 3) + (unsigned long long)lane) << shift);
+    const int up = __shfl_down_sync(mask, lo, 1, kNodeLanes);
+    const int hi = lane == kNodeLanes - 1 ? b : up;
+    const unsigned full8 = (__ballot_sync(mask, hi > lo) & mask) >> ((threadIdx.x & 31) & ~(kNodeLanes - 1));
+    const int c = __popc(full8);
+    int first = 0;
+    if (lane == 0) first = end + atomicAdd(&tb->next[L], c);
+    first = __shfl_sync(mask, first, 0, kNodeLanes);
+    if ((long long)first + c > cap) {
+        if (lane == 0) atomicOr(&tb->fail, 1);
+        return;
+    }
+    if (hi > lo) {
+        const int at = first + __popc(full8 & ((1u << lane) - 1u));
+        __stcg(node + at, make_int4(lo, hi - lo, -1, 0));
+        parent[at] = i;
+    }
+    if (lane == 0) __stcg(node + i, make_int4(nd.x, nd.y, first, c));
 }
 
-__global__ void k_tree_level(const unsigned long long *__restrict__ keys, int4 *node, int *parent, TreeBuild *tb,
-                             int cap, int leaf_max, int split_levels, const int *__restrict__ box_of, int *root_of)
+GZ_DEV unsigned node_mask() { return ((1u << kNodeLanes) - 1u) << ((threadIdx.x & 31) & ~(kNodeLanes - 1)); }
+
+// Levels from the state's on, while they have at most `limit` nodes, by one
+// cluster. `start`: the root first.
+__global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads)
+    k_tree_top(const unsigned long long *__restrict__ keys, int4 *node, int *parent, TreeBuild *tb, int n, int cap,
+               int leaf_max, int split_levels, const int *__restrict__ box_of, int *root_of, int limit, int start)
 {
-    if (tb->fail) return;
-    const int L = tb->L, beg = tb->level_beg, cnt = tb->level_cnt, end = tb->total;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-        int4 nd = node[beg + i];
-        if (box_of && L == split_levels) root_of[box_of[nd.x]] = beg + i;  // one node per box
-        int bound[9];
-        int c = 0;
-        if ((nd.y > leaf_max || L < split_levels) && L < kBits) {
-            child_bounds(keys, nd.x, nd.x + nd.y, L, bound);
-            for (int d = 0; d < 8; d++) c += bound[d + 1] > bound[d];
+    const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int t = blockIdx.x * kTopThreads + threadIdx.x, lane = t % kNodeLanes;
+    const unsigned mask = node_mask();
+    if (start) {
+        if (t < kBits + 1) tb->next[t] = 0;
+        if (t == 0) {
+            node[0] = make_int4(0, n, -1, 0);
+            parent[0] = -1;
+            tb->fail = 0;
+            tb->done = 0;
         }
-        nd.z = -1;
-        nd.w = 0;
-        if (c > 0) {
-            const int first = end + atomicAdd(&tb->next_cnt, c);
-            if ((long long)first + c > cap) {
-                atomicOr(&tb->fail, 1);
-            } else {
-                int k = 0;
-                for (int d = 0; d < 8; d++) {
-                    if (bound[d + 1] > bound[d]) {
-                        node[first + k] = make_int4(bound[d], bound[d + 1] - bound[d], -1, 0);
-                        parent[first + k] = beg + i;
-                        k++;
-                    }
-                }
-                nd.z = first;
-                nd.w = c;
-            }
-        }
-        node[beg + i] = nd;
+        __threadfence();
+        cl.sync();
+    }
+    int L = start ? 0 : tb->L, beg = start ? 0 : tb->level_beg, cnt = start ? (n > 0 ? 1 : 0) : tb->level_cnt;
+    int total = start ? cnt : tb->total;
+    while (cnt > 0 && cnt <= limit) {
+        for (int i = t / kNodeLanes; i < cnt; i += kTopNodes)
+            split_node(keys, node, parent, tb, beg + i, L, total, cap, leaf_max, split_levels, box_of, root_of, lane, mask);
+        __threadfence();
+        cl.sync();
+        beg = total;
+        cnt = *(volatile int *)&tb->fail ? 0 : *(volatile int *)&tb->next[L];
+        total += cnt;
+        L++;
+    }
+    cl.sync();  // every block has read the state
+    if (t == 0) {
+        tb->L = L;
+        tb->level_beg = beg;
+        tb->level_cnt = cnt;
+        tb->total = total;
     }
 }
 
-__global__ void k_tree_next(TreeBuild *tb)
+__global__ void __launch_bounds__(256) k_tree_level(const unsigned long long *__restrict__ keys, int4 *node, int *parent,
+                                                    TreeBuild *tb, int cap, int leaf_max, int split_levels,
+                                                    const int *__restrict__ box_of, int *root_of)
 {
-    TreeBuild &t = *tb;
-    t.level_beg = t.total;
-    t.level_cnt = t.fail ? 0 : t.next_cnt;
-    t.total += t.level_cnt;
-    t.next_cnt = 0;
-    t.L++;
+    const int L = tb->L, beg = tb->level_beg, cnt = tb->level_cnt, end = tb->total;
+    if (cnt == 0) return;  // (also after a failure)
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % kNodeLanes;
+    for (int i = t / kNodeLanes; i < cnt; i += gridDim.x * blockDim.x / kNodeLanes)
+        split_node(keys, node, parent, tb, beg + i, L, end, cap, leaf_max, split_levels, box_of, root_of, lane,
+                   node_mask());
+    // the last block to finish makes the children the next level
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&tb->done, 1) == (int)gridDim.x - 1) {
+        tb->done = 0;
+        tb->level_beg = end;
+        tb->level_cnt = *(volatile int *)&tb->fail ? 0 : *(volatile int *)&tb->next[L];
+        tb->total = end + tb->level_cnt;
+        tb->L = L + 1;
+    }
 }
 
 // children of one level written at next + cpos[i] (cpos: inclusive scan of nch)
@@ -223,21 +279,25 @@ GZ_DEV void st_cg4(double4 *p, double4 v)
     __stcg((double2 *)p + 1, make_double2(v.z, v.w));
 }
 
-// Bottom-up bounding boxes and h maxima in one launch: a leaf reduces its
-// particles, and the last child to finish (atomic count per parent) reduces
-// the parent's children, and so on to the root. With boxes == 0 only the h
-// maxima (lo.w) are refreshed.
-__global__ void k_tree_up(int n_nodes, const int *__restrict__ n_nodes_dev, const int4 *__restrict__ node,
-                          const int *__restrict__ parent, const double *__restrict__ x, const double *__restrict__ y,
-                          const double *__restrict__ z, const double *__restrict__ h, double4 *lo, double4 *hi,
-                          int *done, int boxes)
+// Bottom-up bounding boxes and h maxima in one launch, eight lanes a node: a leaf
+// reduces its particles, and the last child to finish (atomic count per parent)
+// reduces the parent's children, one per lane, and so on to the root. With
+// boxes == 0 only the h maxima (lo.w) are refreshed.
+__global__ void __launch_bounds__(128) k_tree_up(int n_nodes, const int *__restrict__ n_nodes_dev,
+                                                 const int4 *__restrict__ node, const int *__restrict__ parent,
+                                                 const double *__restrict__ x, const double *__restrict__ y,
+                                                 const double *__restrict__ z, const double *__restrict__ h, double4 *lo,
+                                                 double4 *hi, int *done, int boxes)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (n_nodes_dev ? *n_nodes_dev : n_nodes)) return;
-    const int4 nd = node[i];
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int lane = (int)(t % kNodeLanes);
+    int i = (int)(t / kNodeLanes);
+    if (t / kNodeLanes >= (n_nodes_dev ? *n_nodes_dev : n_nodes)) return;
+    const unsigned mask = node_mask();
+    int4 nd = node[i];
     if (nd.z >= 0) return;  // internal: reduced by its last child
     double4 l = make_double4(1e300, 1e300, 1e300, 0.0), u = make_double4(-1e300, -1e300, -1e300, 0.0);
-    for (int j = nd.x; j < nd.x + nd.y; j++) {
+    for (int j = nd.x + lane; j < nd.x + nd.y; j += kNodeLanes) {
         if (boxes) {
             const double px = x[j], py = y[j], pz = z[j];
             l.x = fmin(l.x, px); l.y = fmin(l.y, py); l.z = fmin(l.z, pz);
@@ -246,26 +306,35 @@ __global__ void k_tree_up(int n_nodes, const int *__restrict__ n_nodes_dev, cons
         const double hv = h[j];
         if (hv > l.w) l.w = hv;
     }
-    if (boxes) { lo[i] = l; hi[i] = u; } else { lo[i].w = l.w; }
-    int p = parent[i];
-    while (p >= 0) {
-        __threadfence();
-        const int4 pn = node[p];
-        if (atomicAdd(done + p, 1) != pn.w - 1) return;
-        __threadfence();
+    for (;;) {
+        if (boxes) {
+            l.x = warp_min(l.x, mask, kNodeLanes); l.y = warp_min(l.y, mask, kNodeLanes);
+            l.z = warp_min(l.z, mask, kNodeLanes);
+            u.x = warp_max(u.x, mask, kNodeLanes); u.y = warp_max(u.y, mask, kNodeLanes);
+            u.z = warp_max(u.z, mask, kNodeLanes);
+        }
+        l.w = warp_max(l.w, mask, kNodeLanes);
+        int p = -1;
+        if (lane == 0) {
+            if (boxes) { st_cg4(lo + i, l); st_cg4(hi + i, u); } else { __stcg(&lo[i].w, l.w); }
+            p = parent[i];
+            if (p >= 0) {
+                __threadfence();
+                const bool last = atomicAdd(done + p, 1) == node[p].w - 1;
+                __threadfence();
+                if (!last) p = -1;
+            }
+        }
+        p = __shfl_sync(mask, p, 0, kNodeLanes);
+        if (p < 0) return;
+        i = p;
+        nd = node[i];
         l = make_double4(1e300, 1e300, 1e300, 0.0);
         u = make_double4(-1e300, -1e300, -1e300, 0.0);
-        for (int c = pn.z; c < pn.z + pn.w; c++) {
-            const double4 cl = ld_cg4(lo + c);
-            if (boxes) {
-                const double4 cu = ld_cg4(hi + c);
-                l.x = fmin(l.x, cl.x); l.y = fmin(l.y, cl.y); l.z = fmin(l.z, cl.z);
-                u.x = fmax(u.x, cu.x); u.y = fmax(u.y, cu.y); u.z = fmax(u.z, cu.z);
-            }
-            l.w = fmax(l.w, cl.w);
+        if (lane < nd.w) {
+            l = ld_cg4(lo + nd.z + lane);
+            if (boxes) u = ld_cg4(hi + nd.z + lane);
         }
-        if (boxes) { st_cg4(lo + p, l); st_cg4(hi + p, u); } else { __stcg(&lo[p].w, l.w); }
-        p = parent[p];
     }
 }
 
@@ -842,18 +911,30 @@ void tree_up(int n_nodes, const int4 *node, const int *parent, const double *x, 
 {
     if (n_nodes <= 0) return;
     cudaMemsetAsync(done, 0, sizeof(int) * (size_t)n_nodes, s);
-    k_tree_up<<<(n_nodes + 127) / 128, 128, 0, s>>>(n_nodes, n_nodes_dev, node, parent, x, y, z, h, lo, hi, done,
-                                                     boxes);
+    k_tree_up<<<(unsigned)(((long long)n_nodes * kNodeLanes + 127) / 128), 128, 0, s>>>(n_nodes, n_nodes_dev, node,
+                                                                                       parent, x, y, z, h, lo, hi, done,
+                                                                                       boxes);
 }
+
+// Launches for wide levels: none for sets whose widest level is a few turns of
+// the cluster; the levels that uniform and strongly clustered sets have above the
+// cluster's limit otherwise. Levels left over (deeper trees) fall to the cluster
+// again, whatever their width.
+static int wide_levels(int n) { return n <= 65536 ? 0 : n <= (1 << 20) ? 5 : 8; }
+
+int tree_build_launches(int n) { return wide_levels(n) ? wide_levels(n) + 2 : 1; }
 
 void tree_build_device(const unsigned long long *keys, int n, int4 *node, int *parent, TreeBuild *tb, int cap,
                        int leaf_max, int split_levels, const int *box_of, int *root_of, int blocks, cudaStream_t s)
 {
-    k_tree_init<<<1, 1, 0, s>>>(tb, node, parent, n);
-    for (int L = 0; L <= kBits; L++) {
-        k_tree_level<<<blocks, 128, 0, s>>>(keys, node, parent, tb, cap, leaf_max, split_levels, box_of, root_of);
-        k_tree_next<<<1, 1, 0, s>>>(tb);
-    }
+    const int wide = wide_levels(n);
+    k_tree_top<<<kTopBlocks, kTopThreads, 0, s>>>(keys, node, parent, tb, n, cap, leaf_max, split_levels, box_of, root_of,
+                                                  wide ? kTopLimit : INT32_MAX, 1);
+    if (!wide) return;
+    for (int k = 0; k < wide; k++)
+        k_tree_level<<<blocks, 256, 0, s>>>(keys, node, parent, tb, cap, leaf_max, split_levels, box_of, root_of);
+    k_tree_top<<<kTopBlocks, kTopThreads, 0, s>>>(keys, node, parent, tb, n, cap, leaf_max, split_levels, box_of, root_of,
+                                                  INT32_MAX, 0);
 }
 
 template <bool SYM, bool FILL, bool SOLO>

@@ -26,6 +26,7 @@ void tree_up(int n_nodes, const int4 *node, const int *parent, const double *x, 
 // the device: total nodes, fail when cap would be passed)
 void tree_build_device(const unsigned long long *keys, int n, int4 *node, int *parent, TreeBuild *tb, int cap,
                        int leaf_max, int split_levels, const int *box_of, int *root_of, int blocks, cudaStream_t s);
+int tree_build_launches(int n);  // kernels of one tree_build_device
 void walk_rows(const Tree &t, const double *x, const double *y, const double *z, const double *reach,
                const double *hsym, int symmetric, const int *targets, int n_targets, long long *counts,
                const long long *off, int *nbr, int cap, DevStatus *st, int *next_group, cudaStream_t s);

@@ -71,7 +71,9 @@ struct Tree {
 
 // Device state of the octree build (tree_build_device).
 struct TreeBuild {
-    int level_beg, level_cnt, next_cnt, total, fail, L;
+    int level_beg, level_cnt, total, fail, L;
+    int done;      // blocks of a level's launch that have finished
+    int next[22];  // children made by each level
 };
 
 // What a density row reads of each neighbour, in one 64-byte record (sorted
