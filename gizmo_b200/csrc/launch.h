@@ -47,7 +47,10 @@ long long walk_group_warps();
 // 17.1 and 18.2 at a 16th and a 64th). Symmetric rows are only walked for
 // active lists, whose targets lie in the same dense regions: a 16th (1% of 2M
 // particles active: gradient stage 0.84 against 1.03 ms at a quarter, 1.02 at
-// all; 10% of 1M: 1.29 ms, 2.70 at all).
+// all; 10% of 1M: 1.29 ms, 2.70 at all). While the targets themselves fill the
+// warps at most kSoloWaves times, whatever their density, one warp per target is
+// faster too: a group's walk is one serial chain of ~100 us (density stage of 4,096
+// / 9,261 / 17,576 lattice cells 0.31 / 0.39 / 0.46 ms, as groups 0.38 / 0.47 / 0.47).
 constexpr int kSoloWaves = 4;
 __host__ __device__ inline bool walk_one_target_per_warp(long long n_targets, long long n_particles,
                                                          long long group_warps, bool symmetric)

@@ -693,12 +693,12 @@ GZ_DEV void push_refine(const RefineQueue &q, bool fragile, long long e, long lo
 // Resident 128-thread blocks per multiprocessor the pair kernels ask of the
 // register allocator. Every pair once: FP32 five (at most 96 registers; force
 // stage of 2M lognormal / Plummer particles 9.97 / 6.12 ms, at four, six and seven
-// 10.85 / 6.58, 10.08 / 6.11, 10.03 / 6.07), FP64 three (1.41 ms for 110,003
-// lognormal particles, 1.55 at four, 1.74 at five; 7.07, 7.07 and 7.13 ms for a
-// million Plummer particles). Row entries of a subset read both sides' records
+// 10.85 / 6.58, 10.08 / 6.11, 10.03 / 6.07), FP64 four (7.14 ms for a million
+// Plummer particles, 7.37 at three; 1.33 and 1.35 ms for 110,003 lognormal ones;
+// five 7.13 and 1.74 ms, before the rows per warp followed the size). Row entries of a subset read both sides' records
 // per lane: FP32 four (1% of 2M: 0.69 ms, 0.74 at five), FP64 three (10% of 1M:
 // 1.61 ms, 1.62 at two, 1.81 at four).
-template <typename T> constexpr int kForcePairsMinBlocks = sizeof(T) == 4 ? 5 : 3;
+template <typename T> constexpr int kForcePairsMinBlocks = sizeof(T) == 4 ? 5 : 4;
 template <typename T> constexpr int kForceEntriesMinBlocks = sizeof(T) == 4 ? 4 : 3;
 
 // Pairs that the first attempt at the face does not settle -- the exact Riemann
