@@ -27,13 +27,29 @@ struct DevBuf {
 };
 
 // Search radius of the density rows, as a factor of h (the pair body re-filters
-// r < h exactly, so any factor >= 1 gives the same sums). The reference's runner
-// uses 1.3 (DensitySpec::mode_a_csr_buffer_factor, density_loop.h:316). From a
-// previous step's h the first rows need less: 1.15 x h holds the whole iteration
-// of ~98.6% of particles (Plummer mixture) at 0.66 x the candidates of 1.3 x h;
-// a particle whose h outgrows its row gets a new one at 1.3 x its new h.
-constexpr double kDensityBufferFirst = 1.15;
-constexpr double kDensityBuffer = 1.3;
+// r < h exactly, so any factor >= 1 gives the same sums; the reference's runner
+// uses 1.3, DensitySpec::mode_a_csr_buffer_factor, density_loop.h:316). A particle
+// whose h outgrows its row gets a new one at `regrow` x its new h. Every sum of
+// the iteration pays for the candidates beyond h (1.52 x as many at 1.15 h, 1.16 x
+// at 1.05 h), a row that is outgrown for one more walk of its own. Density stage
+// of 2M particles in ms, (first, regrow):
+//                     1.15,1.3  1.15,1.1  1.10,1.07  1.07,1.04  1.05,1.03  1.03,1.02
+//   Plummer, noisy h      24.4      21.4       19.6       18.6       (17.0)     (16.3)
+//   Plummer, h +-5%        -        14.4       13.2       12.6       (12.0)     (12.3)
+//   lognormal, noisy h    19.5      16.9       15.9       15.4       (14.9)     (14.7)
+//   lognormal, h +-5%      -        12.6       11.7       11.3       (11.6)     (12.0)
+// (in brackets: with the shape sums taken apart from the flow sums, which is worth
+// 1.3 and 0.4 ms at 1.07,1.04). Up to kSmallTargets the extra walks' latency costs
+// more than the candidates: 32,768 lattice cells at h +-5% take 0.47 ms with rows
+// that hold the whole iteration and 0.56 ms at 1.05.
+struct RowFactors {
+    double first, regrow;
+};
+constexpr long long kSmallTargets = 65536;
+constexpr RowFactors row_factors(long long targets)
+{
+    return targets <= kSmallTargets ? RowFactors{1.15, 1.10} : RowFactors{1.05, 1.03};
+}
 
 }  // namespace
 
@@ -1324,7 +1340,8 @@ __global__ void k_g_tree_check(const TreeBuild *tb, GraphState *gs)
 
 int density_caps(const gz_context *c, int *cap0, int *cap1)
 {
-    const double fs[2] = {kDensityBufferFirst, kDensityBuffer};
+    const RowFactors rf = row_factors(c->n);
+    const double fs[2] = {rf.first, rf.regrow};
     int *out[2] = {cap0, cap1};
     for (int k = 0; k < 2; k++) {
         const double f = fs[k];
@@ -1351,7 +1368,7 @@ int graph_buffers(gz_context *c, long long *sym_cap, long long *rq_cap, bool wit
     const size_t N = (size_t)std::max(n, 1);
     int cap0 = 0, cap1 = 0;
     density_caps(c, &cap0, &cap1);
-    const long long nbr_need = (long long)n * cap0 + std::max<long long>(n / 8, 4096) * cap1;
+    const long long nbr_need = (long long)n * cap0 + std::max<long long>(n / 2, 4096) * cap1;
     if (nbr_need > (long long)INT32_MAX * 4) return kNoRoom;
     const long long sc = c->pairs_symmetric + c->pairs_symmetric / 4 + 1024;
     const int mixed = c->prm.precision == GZ_PRECISION_MIXED;
@@ -1497,7 +1514,7 @@ int capture_density_iteration(gz_context *c, cudaStream_t s, cudaGraphConditiona
     const int blocks = c->sms * 8;
     k_g_prep<<<1, 1, 0, s>>>(gs, cap0, cap1, c->d_nbr_cap, n, walk_group_warps(), c->sms);
     k_g_row_radius<<<blocks, 256, 0, s>>>(gs, ptr<int>(c->targets), ptr<int>(c->grow), ptr<double>(c->h),
-                                          kDensityBufferFirst, kDensityBuffer, ptr<double>(c->h_built));
+                                          row_factors(n).first, row_factors(n).regrow, ptr<double>(c->h_built));
     walk_rows_graph(t, ptr<double>(c->x), ptr<double>(c->y), ptr<double>(c->z), ptr<double>(c->h_built),
                     ptr<int>(c->targets), ptr<int>(c->grow), gs, ptr<long long>(c->counts), ptr<int>(c->d_nbr),
                     ptr<DevStatus>(c->status), s);
@@ -2071,12 +2088,11 @@ int gz_hydro_density(gz_context *c, const int *active, int n_active)
     int iter = 0;
     for (iter = 0; iter < kMaxIter && n_todo > 0; iter++) {
         if (n_grow > 0) {
-            k_row_radius<<<(n_grow + 255) / 256, 256, 0, s>>>(n_grow, grow, ptr<double>(c->h),
-                                                               iter == 0 ? kDensityBufferFirst : kDensityBuffer,
+            const double f = iter == 0 ? row_factors(na).first : row_factors(na).regrow;
+            k_row_radius<<<(n_grow + 255) / 256, 256, 0, s>>>(n_grow, grow, ptr<double>(c->h), f,
                                                                ptr<double>(c->h_built));
             c->launches++;
             // slots per padded row: row_slots (2.5 by default) x the expected row length, in multiples of 32
-            const double f = iter == 0 ? kDensityBufferFirst : kDensityBuffer;
             const int cap = std::max(
                 32, std::min(4096, 32 * (int)std::ceil(c->row_slots * c->prm.des_num_ngb * f * f * f / 32.0)));
             long long used = 0, entries = 0;
