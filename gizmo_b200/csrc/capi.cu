@@ -34,12 +34,12 @@ struct DevBuf {
 // at 1.05 h), a row that is outgrown for one more walk of its own. Density stage
 // of 2M particles in ms, (first, regrow):
 //                     1.15,1.3  1.15,1.1  1.10,1.07  1.07,1.04  1.05,1.03  1.03,1.02
-//   Plummer, noisy h      24.4      21.4       19.6       18.6       (17.0)     (16.3)
-//   Plummer, h +-5%        -        14.4       13.2       12.6       (12.0)     (12.3)
-//   lognormal, noisy h    19.5      16.9       15.9       15.4       (14.9)     (14.7)
-//   lognormal, h +-5%      -        12.6       11.7       11.3       (11.6)     (12.0)
-// (in brackets: with the shape sums taken apart from the flow sums, which is worth
-// 1.3 and 0.4 ms at 1.07,1.04). Up to kSmallTargets the extra walks' latency costs
+//   Plummer, noisy h      24.4      21.4       19.6       18.6        18.2      (16.3)
+//   Plummer, h +-5%        -        14.4       13.2       12.6        12.5      (12.3)
+//   lognormal, noisy h    19.5      16.9       15.9       15.4        15.3      (14.7)
+//   lognormal, h +-5%      -        12.6       11.7       11.3        11.5      (12.0)
+// (in brackets: with the shape sums taken apart from the flow sums, seven blocks per
+// multiprocessor, where 1.05,1.03 took 17.0, 12.0, 14.9 and 11.6). Up to kSmallTargets the extra walks' latency costs
 // more than the candidates: 32,768 lattice cells at h +-5% take 0.47 ms with rows
 // that hold the whole iteration and 0.56 ms at 1.05.
 struct RowFactors {
@@ -1338,6 +1338,23 @@ __global__ void k_g_tree_check(const TreeBuild *tb, GraphState *gs)
     if (tb->fail) gs->fail |= kGraphFailTree;
 }
 
+// the flow sums of the na targets of a density pass, at their converged lengths
+// (captured: not taken once the graph has failed)
+void flow_sums(gz_context *c, int na, bool captured, cudaStream_t s)
+{
+    DensityWork w{};
+    w.gs = captured ? ptr<GraphState>(c->gstate) : nullptr;
+    w.todo = ptr<int>(c->targets);
+    w.n_todo = na;
+    w.beg = ptr<long long>(c->d_beg);
+    w.end = ptr<long long>(c->d_end);
+    w.nbr = ptr<int>(c->d_nbr);
+    w.rec = ptr<DensRec>(c->rec);
+    w.acc = ptr<double>(c->acc);
+    // (not under GZ_TIMER_DENSITY_SUMS, which counts the iteration's rows)
+    density_sums(c->pp, view(c), w, DensitySums::flow, lanes_per_row(c, na, 4), s);
+}
+
 int density_caps(const gz_context *c, int *cap0, int *cap1)
 {
     const RowFactors rf = row_factors(c->n);
@@ -1657,6 +1674,7 @@ int graph_capture(gz_context *c, long long sym_cap, long long rq_cap, bool with_
         if ((rc = add_conditional(c, s, h_loop, cudaGraphCondTypeWhile, &body_loop))) break;
         if ((rc = body(s1, body_loop, [&] { return capture_density_iteration(c, s1, h_loop); }))) break;
         if ((rc = check_last(c, "density iteration"))) break;
+        flow_sums(c, n, true, s);
         density_finalize(c->pp, ps, ptr<double>(c->acc), ptr<int>(c->targets), n, s);
         if ((rc = make_handle(c, s, &h_conv, 0))) break;
         k_g_if_converged<<<1, 1, 0, s>>>(ptr<GraphState>(c->gstate), h_conv);
@@ -1684,13 +1702,13 @@ int graph_capture(gz_context *c, long long sym_cap, long long rq_cap, bool with_
     c->g.graph = g;
     if (check_last(c, "end of capture")) { graph_release(c); return c->err; }
     // this library's kernels in each part (the key sort and scans are CUB's):
-    // setup (targets, active flags, prep, pack, state) + finalize + the
+    // setup (targets, active flags, prep, pack, state) + flow sums + finalize + the
     // convergence test; per iteration prep, radii, two walk modes, padded
     // rows, overflow check, overflow walk, three sums instances, after_iter,
     // the selection's three steps, next; the rows' split, counts and check;
     // scatter, sort, the gradient pack and rows, the force preloop, pack,
     // pairs, deferred pairs, (refine,) gather, finish
-    c->g.kernels_top = 7 + restage_kernels;
+    c->g.kernels_top = 8 + restage_kernels;
     c->g.kernels_loop = 15;
     c->g.kernels_sym = 3;
     c->g.kernels_tail = c->prm.precision == GZ_PRECISION_MIXED ? 11 : 10;
@@ -2118,8 +2136,7 @@ int gz_hydro_density(gz_context *c, const int *active, int n_active)
         GZ_CUDA(c, cudaMemsetAsync(c->flag.p, 0, sizeof(int), s));
         const EventPair *ev = timer_launch(c, GZ_TIMER_DENSITY_SUMS, w.n_todo);
         ev_start(ev, s);
-        if (c->prm.precision == GZ_PRECISION_MIXED) density_sums_mixed(c->pp, ps, w, lanes_per_row(c, w.n_todo, 4), s);
-        else density_sums_fp64(c->pp, ps, w, lanes_per_row(c, w.n_todo, 4), s);
+        density_sums(c->pp, ps, w, DensitySums::shape, lanes_per_row(c, w.n_todo, 4), s);
         ev_stop(ev, s);
         density_after_iter(c->pp, ps, w, ptr<DevStatus>(c->status), s);
         c->launches += 2;
@@ -2150,6 +2167,8 @@ int gz_hydro_density(gz_context *c, const int *active, int n_active)
     }
     c->last_iters = iter;
     c->d_used = base;
+    flow_sums(c, na, false, s);
+    c->launches++;
     density_finalize(c->pp, ps, ptr<double>(c->acc), ptr<int>(c->targets), na, s);
     if (na > 0) c->launches++;
     GZ_CUDA(c, cudaGetLastError());
@@ -2572,8 +2591,7 @@ int gz_density_sums(gz_context *c, const int *active, int n_active, double *acc,
     w.acc = ptr<double>(c->acc);
     const EventPair *ev = timer_launch(c, GZ_TIMER_DENSITY_SUMS, w.n_todo);
     ev_start(ev, s);
-    if (c->prm.precision == GZ_PRECISION_MIXED) density_sums_mixed(c->pp, ps, w, lanes_per_row(c, w.n_todo, 4), s);
-    else density_sums_fp64(c->pp, ps, w, lanes_per_row(c, w.n_todo, 4), s);
+    density_sums(c->pp, ps, w, DensitySums::all, lanes_per_row(c, w.n_todo, 4), s);
     ev_stop(ev, s);
     GZ_CUDA(c, cudaGetLastError());
     const int n = c->n;

@@ -94,6 +94,7 @@ struct DensityWork {
     int *rebuild;           // set when any radius outgrows its row
     unsigned long long *h_iter_max;  // atomic maximum of every radius the iteration moves to (double bits)
     int iter;
+    const GraphState *gs;   // captured pass: the rows are not all there when it failed (null: a plain pass)
 };
 
 // passes_fp64.cu / passes_mixed.cu (same kernels, pair arithmetic double / float)
@@ -102,8 +103,10 @@ struct PassLaunch {
 };
 
 void density_pack(const Particles &ps, DensRec *rec, cudaStream_t s);
-void density_sums_fp64(const PassParams &p, const Particles &ps, const DensityWork &w, int tpt, cudaStream_t s);
-void density_sums_mixed(const PassParams &p, const Particles &ps, const DensityWork &w, int tpt, cudaStream_t s);
+// the sums of w.todo's rows: all 17, the ones the iteration decides on, or the others
+enum class DensitySums { all, shape, flow };
+void density_sums(const PassParams &p, const Particles &ps, const DensityWork &w, DensitySums what, int tpt,
+                  cudaStream_t s);
 void density_after_iter(const PassParams &p, const Particles &ps, const DensityWork &w, DevStatus *st, cudaStream_t s);
 // Captured-pass forms (GraphState): every TPT instance is launched with `blocks`
 // blocks and the one the device state names runs; after_iter writes the

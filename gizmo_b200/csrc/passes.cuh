@@ -50,32 +50,49 @@ template <typename R> GZ_DEV R ldg_record(const R *__restrict__ p)
     return r;
 }
 
+// Which of a density row's 17 sums a pass takes. The kernel-length iteration only
+// decides on the shape sums (the count, DrkernNgb, NV_T and the face sums:
+// after_iter), which need no more than the 32 bytes of position and mass of a
+// neighbour, 13 of the sums' registers and no division; the flow sums (Rho, DivVel,
+// ParticleVel) are taken once, at the converged length. Density stage of 2M Plummer
+// / lognormal particles 16.4 / 14.4 ms against 18.2 / 15.3 with all 17 sums in every
+// iteration, of a million Plummer ones 10.8 against 12.1 (10 to 12 iterations of
+// ever fewer rows, the sums of about four full ones); from h +-5% 11.7 / 11.1 ms
+// against 12.5 / 11.5.
+enum : int { kSumsAll = 0, kSumsShape = 1, kSumsFlow = 2 };
+
 // A neighbour's density record through the read-only data path, in 16-byte
-// pieces, without its padding word.
-GZ_DEV DensRec load_dens_rec(const DensRec *__restrict__ rec, int j)
+// pieces: without its padding word, and without the velocity for the shape sums.
+template <int WHAT> GZ_DEV DensRec load_dens_rec(const DensRec *__restrict__ rec, int j)
 {
     const double2 *q = reinterpret_cast<const double2 *>(rec + j);
-    const double2 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2);
+    const double2 q0 = __ldg(q), q1 = __ldg(q + 1);
     DensRec r;
-    r.x = q0.x; r.y = q0.y; r.z = q1.x; r.m = q1.y; r.vx = q2.x; r.vy = q2.y;
-    r.vz = __ldg(reinterpret_cast<const double *>(q + 3));
-    r.pad = 0.0;
+    r.x = q0.x; r.y = q0.y; r.z = q1.x; r.m = q1.y;
+    r.vx = r.vy = r.vz = r.pad = 0.0;
+    if (WHAT != kSumsShape) {
+        const double2 q2 = __ldg(q + 2);
+        r.vx = q2.x; r.vy = q2.y;
+        r.vz = __ldg(reinterpret_cast<const double *>(q + 3));
+    }
     return r;
 }
 
 // The sums of target t's density row, by the TPT lanes (`lane` of them, on
 // `mask`) that own it; lane 0 stores them.
-template <typename T, int TPT>
+template <typename T, int TPT, int WHAT>
 GZ_DEV void density_row(const PassParams &p, const Particles &ps, const DensityWork &w, int t, int lane,
                         unsigned mask)
 {
+    constexpr bool kShape = WHAT != kSumsFlow, kFlow = WHAT != kSumsShape;
     const double xi = ps.x[t], yi = ps.y[t], zi = ps.z[t];
     const double hd = ps.h[t];
     const double h2 = hd * hd;
     const T h = T(hd);
     T hinv, hinv3, hinv4;
     k_hinv(h, hinv, hinv3, hinv4);
-    const T vix = T(ps.vx[t]), viy = T(ps.vy[t]), viz = T(ps.vz[t]);
+    T vix = T(0), viy = T(0), viz = T(0);
+    if (kFlow) { vix = T(ps.vx[t]); viy = T(ps.vy[t]); viz = T(ps.vz[t]); }
     const int mfv = p.method == 1;
     double a[17];
 #pragma unroll
@@ -91,39 +108,44 @@ GZ_DEV void density_row(const PassParams &p, const Particles &ps, const DensityW
         const T u = r * hinv;
         T wk, dwk;
         k_main(p.kernel, u, hinv3, hinv4, wk, dwk);
-        const T mj = T(mjd);
-        const T mj_wk = mj * wk;
-        a[0] += (double)wk;
-        a[1] += (double)mj_wk;
+        const T mj_wk = T(mjd) * wk;
         const T vjx = T(rj.vx), vjy = T(rj.vy), vjz = T(rj.vz);
-        if (mfv && r == T(0)) {
-            a[14] += (double)(mj_wk * vjx);
-            a[15] += (double)(mj_wk * vjy);
-            a[16] += (double)(mj_wk * vjz);
+        if (kShape) a[0] += (double)wk;
+        if (kFlow) {
+            a[1] += (double)mj_wk;
+            if (mfv && r == T(0)) {
+                a[14] += (double)(mj_wk * vjx);
+                a[15] += (double)(mj_wk * vjy);
+                a[16] += (double)(mj_wk * vjz);
+            }
         }
-        a[2] += (double)(-(T(3) * hinv * wk + u * dwk));
+        if (kShape) a[2] += (double)(-(T(3) * hinv * wk + u * dwk));
         if (r > T(0)) {
             const T px = T(dx), py = T(dy), pz = T(dz);
-            a[4] += (double)(px * px * wk);
-            a[5] += (double)(py * py * wk);
-            a[6] += (double)(pz * pz * wk);
-            a[7] += (double)(px * py * wk);
-            a[8] += (double)(py * pz * wk);
-            a[9] += (double)(px * pz * wk);
-            a[10] += (double)(wk * px);
-            a[11] += (double)(wk * py);
-            a[12] += (double)(wk * pz);
-            const T dvx = vix - vjx, dvy = viy - vjy, dvz = viz - vjz;
-            if (mfv) {
-                a[14] += (double)(mj_wk * (vix - dvx));
-                a[15] += (double)(mj_wk * (viy - dvy));
-                a[16] += (double)(mj_wk * (viz - dvz));
+            if (kShape) {
+                a[4] += (double)(px * px * wk);
+                a[5] += (double)(py * py * wk);
+                a[6] += (double)(pz * pz * wk);
+                a[7] += (double)(px * py * wk);
+                a[8] += (double)(py * pz * wk);
+                a[9] += (double)(px * pz * wk);
+                a[10] += (double)(wk * px);
+                a[11] += (double)(wk * py);
+                a[12] += (double)(wk * pz);
             }
-            a[3] -= (double)(dwk * (px * dvx + py * dvy + pz * dvz) / r);
+            if (kFlow) {
+                const T dvx = vix - vjx, dvy = viy - vjy, dvz = viz - vjz;
+                if (mfv) {
+                    a[14] += (double)(mj_wk * (vix - dvx));
+                    a[15] += (double)(mj_wk * (viy - dvy));
+                    a[16] += (double)(mj_wk * (viz - dvz));
+                }
+                a[3] -= (double)(dwk * (px * dvx + py * dvy + pz * dvz) / r);
+            }
         }
     };
     // one record in flight per lane: the register budget goes to resident
-    // warps (six 128-thread blocks per multiprocessor), which hide the
+    // warps (kDensityBlocks of 128 threads per multiprocessor), which hide the
     // gather latency better than a second record per lane does; the next
     // entry's index is loaded a step ahead, so the record load does not wait
     // on it
@@ -134,26 +156,35 @@ GZ_DEV void density_row(const PassParams &p, const Particles &ps, const DensityW
     for (; e < b1; e += TPT) {
         const long long en = e + TPT;
         const int jn = en < b1 ? __ldg(nbr + en) : 0;
-        pair(load_dens_rec(w.rec, j));
+        pair(load_dens_rec<WHAT>(w.rec, j));
         j = jn;
     }
+    const size_t n = (size_t)ps.n;
 #pragma unroll
-    for (int k = 0; k < 17; k++) a[k] = warp_sum(a[k], mask, TPT);
-    if (lane == 0) {
-        const size_t n = (size_t)ps.n;
-#pragma unroll
-        for (int k = 0; k < 17; k++) w.acc[k * n + t] = a[k];
+    for (int k = 0; k < 17; k++) {
+        const bool flow = k == 1 || k == 3 || k >= 14;
+        if (k == 13 || (flow ? !kFlow : !kShape)) continue;
+        a[k] = warp_sum(a[k], mask, TPT);
+        if (lane == 0) w.acc[k * n + t] = a[k];
     }
 }
 
-template <typename T, int TPT>
-__global__ void __launch_bounds__(kDensityBlock, 6) k_density_sums(PassParams p, Particles ps, DensityWork w)
+// Resident 128-thread blocks per multiprocessor the density sums ask of the
+// register allocator: shape and flow sums eight (at most 64 registers; density
+// stage of 2M Plummer / lognormal particles 16.4 / 14.3 ms, at six, seven and nine
+// 17.7 / 15.4, 17.0 / 14.9 and 16.7 / 14.6), all 17 sums six (at eight 58 against
+// 49 ms for the sums of 256^3).
+template <int WHAT> constexpr int kDensityBlocks = WHAT == kSumsAll ? 6 : 8;
+
+template <typename T, int TPT, int WHAT>
+__global__ void __launch_bounds__(kDensityBlock, kDensityBlocks<WHAT>) k_density_sums(PassParams p, Particles ps,
+                                                                                      DensityWork w)
 {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int slot = gtid / TPT, lane = gtid % TPT;
-    if (slot >= w.n_todo) return;
+    if (slot >= w.n_todo || (w.gs && w.gs->fail)) return;
     const unsigned mask = (TPT == 32) ? 0xffffffffu : (((1u << TPT) - 1u) << ((threadIdx.x & 31) & ~(TPT - 1)));
-    density_row<T, TPT>(p, ps, w, w.todo[slot], lane, mask);
+    density_row<T, TPT, WHAT>(p, ps, w, w.todo[slot], lane, mask);
 }
 
 // The same rows for a captured pass: the iteration's target count and lane
@@ -165,9 +196,8 @@ __global__ void __launch_bounds__(kDensityBlock, 6) k_density_sums(PassParams p,
 // is not the iteration's returns at once. Each row is summed by the same
 // lanes in the same order as k_density_sums sums it.
 template <typename T, int TPT>
-__global__ void __launch_bounds__(kDensityBlock, 6) k_density_sums_graph(PassParams p, Particles ps, DensityWork w,
-                                                                         GraphState *gs,
-                                                                         const int *__restrict__ todo)
+__global__ void __launch_bounds__(kDensityBlock, kDensityBlocks<kSumsShape>)
+    k_density_sums_graph(PassParams p, Particles ps, DensityWork w, GraphState *gs, const int *__restrict__ todo)
 {
     __shared__ int s_chunk;
     if (gs->fail || gs->tpt != TPT) return;
@@ -182,21 +212,20 @@ __global__ void __launch_bounds__(kDensityBlock, 6) k_density_sums_graph(PassPar
         __syncthreads();  // read by every thread before the next draw
         if ((long long)chunk * kRows >= n_todo) break;
         const int slot = chunk * kRows + (int)threadIdx.x / TPT;
-        if (slot < n_todo) density_row<T, TPT>(p, ps, w, todo[slot], lane, mask);
+        if (slot < n_todo) density_row<T, TPT, kSumsShape>(p, ps, w, todo[slot], lane, mask);
     }
 }
 
-template <typename T>
+template <typename T, int WHAT>
 void launch_density_sums(const PassParams &p, const Particles &ps, const DensityWork &w, int tpt, cudaStream_t s)
 {
     if (w.n_todo <= 0) return;
     const long long threads = (long long)w.n_todo * tpt;
     const unsigned blocks = (unsigned)((threads + kDensityBlock - 1) / kDensityBlock);
     switch (tpt) {
-        case 4: k_density_sums<T, 4><<<blocks, kDensityBlock, 0, s>>>(p, ps, w); break;
-        case 8: k_density_sums<T, 8><<<blocks, kDensityBlock, 0, s>>>(p, ps, w); break;
-        case 32: k_density_sums<T, 32><<<blocks, kDensityBlock, 0, s>>>(p, ps, w); break;
-        default: k_density_sums<T, 16><<<blocks, kDensityBlock, 0, s>>>(p, ps, w); break;
+        case 4: k_density_sums<T, 4, WHAT><<<blocks, kDensityBlock, 0, s>>>(p, ps, w); break;
+        case 8: k_density_sums<T, 8, WHAT><<<blocks, kDensityBlock, 0, s>>>(p, ps, w); break;
+        default: k_density_sums<T, 16, WHAT><<<blocks, kDensityBlock, 0, s>>>(p, ps, w); break;
     }
 }
 

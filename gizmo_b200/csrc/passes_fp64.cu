@@ -31,9 +31,20 @@ void density_pack(const Particles &ps, DensRec *rec, cudaStream_t s)
         k_pack_density<<<(ps.n + kPackBlock - 1) / kPackBlock, kPackBlock, kPackBlock * sizeof(DensRec), s>>>(ps, rec);
 }
 
-void density_sums_fp64(const PassParams &p, const Particles &ps, const DensityWork &w, int tpt, cudaStream_t s)
+// The density sums feed the bracketed kernel-length iteration, whose
+// accept/bracket decisions are discontinuous in NumNgb, DrkernNgb, NV_T and
+// the face weights: computing them in FP32 moves the converged h of any
+// particle whose count sits within ~1e-7 of a band edge by up to the band
+// width (~1e-3). Both forms therefore take them in FP64 and converge to
+// identical h.
+void density_sums(const PassParams &p, const Particles &ps, const DensityWork &w, DensitySums what, int tpt,
+                  cudaStream_t s)
 {
-    launch_density_sums<double>(p, ps, w, tpt, s);
+    switch (what) {
+        case DensitySums::all: launch_density_sums<double, kSumsAll>(p, ps, w, tpt, s); break;
+        case DensitySums::shape: launch_density_sums<double, kSumsShape>(p, ps, w, tpt, s); break;
+        case DensitySums::flow: launch_density_sums<double, kSumsFlow>(p, ps, w, tpt, s); break;
+    }
 }
 
 void density_sums_graph(const PassParams &p, const Particles &ps, const DensityWork &w, GraphState *gs,
