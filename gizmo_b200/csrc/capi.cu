@@ -71,6 +71,7 @@ struct gz_context {
     bool have_bins = false;          // timebin (and vsig) were uploaded
     bool binact_on = false;          // gz_set_bin_active gave a table
     DevBuf dl;                       // download staging, [9][n] doubles (widest output field)
+    void *pinned = nullptr;          // page-locked staging of small downloads
     DevBuf rec;                      // packed neighbour records of the running pass
     DevBuf work;                     // work counter of the persistent walks
     long long launches = 0;          // kernels of this library launched by the context
@@ -1865,6 +1866,7 @@ int gz_destroy(gz_context *c)
         for (cudaEvent_t e : {c->ev_in_free, c->ev_in_done, c->ev_out_ready, c->ev_out_done}) cudaEventDestroy(e);
     }
     for (DevBuf *b : all_buffers(c)) release(*b);
+    if (c->pinned) cudaFreeHost(c->pinned);
     for (auto &t : c->timers)
         for (auto &e : t.ev) { cudaEventDestroy(e.start); cudaEventDestroy(e.stop); }
     cudaStreamDestroy(c->stream);
@@ -2413,10 +2415,24 @@ static void scatter_fields(gz_context *c, const std::vector<OutField> &f, size_t
     }
 }
 
+// The page-locked buffer of small downloads (made on first use, freed with the
+// context); false when it cannot be had.
+constexpr size_t kPinnedBytes = 4 << 20;
+static bool pinned_buffer(gz_context *c)
+{
+    if (!c->pinned && cudaHostAlloc(&c->pinned, kPinnedBytes, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        c->pinned = nullptr;
+    }
+    return c->pinned != nullptr;
+}
+
 // gz_download into host arrays through the staging buffer, or (to_device)
 // straight into the caller's device arrays (gz_download_device). The host
 // form scatters as many fields as the staging holds (up to 16 doubles per
-// particle), copies them out and waits once per such group.
+// particle), copies them out and waits once per such group: small groups in one copy
+// into page-locked memory, from where the host hands them out (a copy of a few KB
+// into pageable memory costs ~10 us, and there are 19 fields).
 static int download_to(gz_context *c, const gz_outputs *o, bool to_device)
 {
     if (!c || !o) return GZ_ERR_ARG;
@@ -2436,7 +2452,7 @@ static int download_to(gz_context *c, const gz_outputs *o, bool to_device)
         GZ_CUDA(c, cudaStreamSynchronize(s));
         return GZ_OK;
     }
-    const size_t cap = sizeof(double) * 16 * (size_t)n;
+    const size_t cap = sizeof(double) * std::max<size_t>(16 * (size_t)n, std::min<size_t>(48 * (size_t)n, kPinnedBytes / 8));
     if (ensure(c, c->dl, cap + 64)) return c->err;
     for (size_t first = 0; first < f.size();) {
         std::vector<void *> at;
@@ -2450,6 +2466,15 @@ static int download_to(gz_context *c, const gz_outputs *o, bool to_device)
         }
         scatter_fields(c, f, first, last, s, at);
         GZ_CUDA(c, cudaGetLastError());
+        if (used <= kPinnedBytes && pinned_buffer(c)) {
+            GZ_CUDA(c, cudaMemcpyAsync(c->pinned, c->dl.p, used, cudaMemcpyDeviceToHost, s));
+            GZ_CUDA(c, cudaStreamSynchronize(s));
+            for (size_t i = first; i < last; i++)
+                memcpy(f[i].dst, (char *)c->pinned + ((char *)at[i - first] - (char *)c->dl.p),
+                       (size_t)f[i].bytes * f[i].k * n);
+            first = last;
+            continue;
+        }
         for (size_t i = first; i < last; i++)
             GZ_CUDA(c, cudaMemcpyAsync(f[i].dst, at[i - first], (size_t)f[i].bytes * f[i].k * n, cudaMemcpyDeviceToHost, s));
         GZ_CUDA(c, cudaStreamSynchronize(s));
