@@ -51,6 +51,8 @@ constexpr RowFactors row_factors(long long targets)
     return targets <= kSmallTargets ? RowFactors{1.15, 1.10} : RowFactors{1.05, 1.03};
 }
 
+constexpr double kRowSlots = 2.5;  // default padded density-row slots per expected row entry
+
 }  // namespace
 
 struct gz_context {
@@ -117,7 +119,7 @@ struct gz_context {
     int sms = 148;                   // multiprocessors of the device
     // walk tuning (gz_tuning): neither changes a result, both change the walk's cost
     int leaf_max = kLeafMax;         // octree leaf size
-    double row_slots = 2.5;          // padded density-row slots per expected row entry
+    double row_slots = kRowSlots;    // padded density-row slots per expected row entry
     // the pass over every particle captured as one CUDA graph (gz_hydro_pass)
     struct Graph {
         cudaGraph_t graph = nullptr;
@@ -150,16 +152,24 @@ namespace {
 // Lanes per row of the density and gradient row kernels. Fewer lanes per row
 // mean more rows in flight per warp and a shorter cross-lane reduction, but
 // fewer threads: the fewest lanes (at least `min_lanes`) with which the rows
-// still give about eight waves of resident threads (2048 per multiprocessor),
-// at most 16. The density rows keep at least 4 lanes: their pair work is long
-// and the lanes of a row share its loads.
-int lanes_per_row(const gz_context *c, long long rows, int min_lanes)
+// still give `waves` waves of resident threads (2048 per multiprocessor), at
+// most 16. The density rows keep at least 4 lanes (their pair work is long and
+// the lanes of a row share its loads) and eight waves (four: 15.7 against 15.5 ms
+// for the density stage of 2M Plummer particles, 10.3 against 10.1 of a million).
+int lanes_per_row(const gz_context *c, long long rows, int min_lanes, int waves)
 {
-    const long long want = (long long)c->sms * 2048 * 8;
+    const long long want = (long long)c->sms * 2048 * waves;
     int tpt = min_lanes;
     while (tpt < 16 && rows * tpt < want) tpt *= 2;
     return tpt;
 }
+int density_lanes(const gz_context *c, long long rows) { return lanes_per_row(c, rows, 4, 8); }
+// Gradient rows: two lanes at least (one: gradient stage 4.36 and 6.32 against 4.10
+// and 6.17 ms for 2M Plummer and lognormal particles, whose rows differ in length)
+// and two waves (1M lattice cells 1.08 ms at two lanes, 1.21 at the four that eight
+// waves asked for; a million Plummer particles 2.63 and 2.59; 110,003 lognormal ones
+// 0.54 at eight, 0.58 at sixteen).
+int gradient_lanes(const gz_context *c, long long rows) { return lanes_per_row(c, rows, 2, 2); }
 
 // The event pair for one launch of timer `id` (null when timing is off, or
 // when no event could be had: that launch then goes untimed).
@@ -1150,7 +1160,7 @@ __global__ void k_g_prep(GraphState *gs, int cap0, int cap1, long long nbr_cap, 
     g.after_next = 0;
     g.extra = 0;
     g.next_group[0] = g.next_group[1] = 0;
-    // lanes per density row: lanes_per_row(n_todo, 4)
+    // lanes per density row: density_lanes(n_todo)
     const long long want = (long long)sms * 2048 * 8;
     int tpt = 4;
     while (tpt < 16 && (long long)g.n_todo * tpt < want) tpt *= 2;
@@ -1367,7 +1377,7 @@ void flow_sums(gz_context *c, int na, bool captured, cudaStream_t s)
     w.rec = ptr<DensRec>(c->rec);
     w.acc = ptr<double>(c->acc);
     // (not under GZ_TIMER_DENSITY_SUMS, which counts the iteration's rows)
-    density_sums(c->pp, view(c), w, DensitySums::flow, lanes_per_row(c, na, 4), s);
+    density_sums(c->pp, view(c), w, DensitySums::flow, density_lanes(c, na), s);
 }
 
 int density_caps(const gz_context *c, int *cap0, int *cap1)
@@ -1613,7 +1623,7 @@ int capture_gradients_force(gz_context *c, cudaStream_t s, long long rq_cap)
     sym_sort(n, ptr<long long>(c->s_off), ptr<int>(c->s_acnt), ptr<int>(c->s_tmp), ptr<int>(c->s_nbr), s);
     Csr rows{ptr<long long>(c->s_off), ptr<int>(c->s_nbr)};
     Particles ps = view(c);
-    gradients_fp64(c->pp, ps, ptr<int>(c->targets), n, rows, lanes_per_row(c, n, 1), c->rec.p, nullptr, s);
+    gradients_fp64(c->pp, ps, ptr<int>(c->targets), n, rows, gradient_lanes(c, n), c->rec.p, nullptr, s);
     if (c->have_bins) GZ_CUDA(c, cudaMemsetAsync(c->wakeup.p, 0, sizeof(int) * N, s));
     force_preloop(c->pp, ps, ptr<int>(c->targets), n, s);
     GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), s));
@@ -2159,7 +2169,7 @@ int gz_hydro_density(gz_context *c, const int *active, int n_active)
         GZ_CUDA(c, cudaMemsetAsync(c->flag.p, 0, sizeof(int), s));
         const EventPair *ev = timer_launch(c, GZ_TIMER_DENSITY_SUMS, w.n_todo);
         ev_start(ev, s);
-        density_sums(c->pp, ps, w, DensitySums::shape, lanes_per_row(c, w.n_todo, 4), s);
+        density_sums(c->pp, ps, w, DensitySums::shape, density_lanes(c, w.n_todo), s);
         ev_stop(ev, s);
         density_after_iter(c->pp, ps, w, ptr<DevStatus>(c->status), s);
         c->launches += 2;
@@ -2229,7 +2239,7 @@ int gz_hydro_gradients(gz_context *c, const int *active, int n_active)
     // record gathers, not by arithmetic (FP32 terms saved 0.6 of 26 ms per step
     // at 256^3), and FP64 gradients make the mixed form's force inputs the FP64
     // form's exactly (FP32 terms left 9 of 16.8M particles above 1e-5).
-    gradients_fp64(c->pp, ps, ptr<int>(c->targets), na, rows, lanes_per_row(c, na, 1), c->rec.p, ev, c->stream);
+    gradients_fp64(c->pp, ps, ptr<int>(c->targets), na, rows, gradient_lanes(c, na), c->rec.p, ev, c->stream);
     if (na > 0) c->launches += 2;  // the record pack and the rows
     GZ_CUDA(c, cudaGetLastError());
     if (read_status(c)) return c->err;
@@ -2637,7 +2647,7 @@ int gz_density_sums(gz_context *c, const int *active, int n_active, double *acc,
     w.acc = ptr<double>(c->acc);
     const EventPair *ev = timer_launch(c, GZ_TIMER_DENSITY_SUMS, w.n_todo);
     ev_start(ev, s);
-    density_sums(c->pp, ps, w, DensitySums::all, lanes_per_row(c, w.n_todo, 4), s);
+    density_sums(c->pp, ps, w, DensitySums::all, density_lanes(c, w.n_todo), s);
     ev_stop(ev, s);
     GZ_CUDA(c, cudaGetLastError());
     const int n = c->n;
@@ -2726,7 +2736,7 @@ int gz_autotune(gz_context *c, gz_tuning *chosen)
         GZ_CUDA(c, cudaEventElapsedTime(&ms, e0, e1));
         return 0;
     };
-    gz_tuning best{c->leaf_max, 0, c->row_slots};
+    gz_tuning best{c->leaf_max, 0, kRowSlots};  // (the leaf sizes are compared at the default slots)
     float best_ms = 1e30f, ms = 0;
     int rc = 0;
     for (int leaf : {32, 64, 96, 128}) {

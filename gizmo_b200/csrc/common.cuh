@@ -45,6 +45,29 @@ GZ_DEV double sep2(double xi, double yi, double zi, double xj, double yj, double
     return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
 }
 
+// The same values for the row sums, which are bound by FP64 issue: nearly every pair
+// lies within half a box on every axis, and a high word below half's says so
+// exactly, in the integer pipe, where sep2's six comparisons are FP64 instructions.
+// Density and gradient stages of 2M lognormal particles 13.5 and 6.2 against 14.3
+// and 6.8 ms, of 2M Plummer ones 15.5 and 4.1 against 16.4 and 4.5, of a million
+// in FP64 10.1 and 2.6 against 10.7 and 2.9. (The pair kernels and the force gather
+// keep sep2: it cost them registers, 10.1 -> 11.0 ms for the force stage of 2M.)
+GZ_DEV double sep2_near(double xi, double yi, double zi, double xj, double yj, double zj, double box, double half,
+                        double &dx, double &dy, double &dz)
+{
+    dx = __dsub_rn(xi, xj);
+    dy = __dsub_rn(yi, yj);
+    dz = __dsub_rn(zi, zj);
+    const int mx = __double2hiint(dx) & 0x7fffffff, my = __double2hiint(dy) & 0x7fffffff;
+    const int mz = __double2hiint(dz) & 0x7fffffff;
+    if (max(max(mx, my), mz) >= __double2hiint(half)) {
+        dx = wrap1(dx, box, half);
+        dy = wrap1(dy, box, half);
+        dz = wrap1(dz, box, half);
+    }
+    return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+}
+
 GZ_DEV uint32_t spread3(uint32_t x)
 {
     x &= 0x3ff;

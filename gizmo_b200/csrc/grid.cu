@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(256, 8) k_sym_split(int n, const double *__res
         if (e < b1) {
             j = nbr[e];
             double dx, dy, dz;
-            const double r2 = sep2(xi, yi, zi, x[j], y[j], z[j], box, half, dx, dy, dz);
+            const double r2 = sep2_near(xi, yi, zi, x[j], y[j], z[j], box, half, dx, dy, dz);
             in_a = (r2 > 0) && (r2 < hi2);
             if (in_a) {
                 const double hj = h[j];

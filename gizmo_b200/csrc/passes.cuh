@@ -102,7 +102,7 @@ GZ_DEV void density_row(const PassParams &p, const Particles &ps, const DensityW
         const double mjd = rj.m;
         if (mjd <= 0) return;
         double dx, dy, dz;
-        const double r2 = sep2(xi, yi, zi, rj.x, rj.y, rj.z, p.box, p.half, dx, dy, dz);
+        const double r2 = sep2_near(xi, yi, zi, rj.x, rj.y, rj.z, p.box, p.half, dx, dy, dz);
         if (r2 >= h2) return;
         const T r = Real<T>::sqrt_(T(r2));
         const T u = r * hinv;
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(128, 4) k_gradients(PassParams p, Particles ps
             if (mj <= 0) continue;
             if (rhoj <= 0 || hjd <= 0) continue;
             double dx, dy, dz;
-            const double r2 = sep2(xi, yi, zi, rj.x, rj.y, rj.z, p.box, p.half, dx, dy, dz);
+            const double r2 = sep2_near(xi, yi, zi, rj.x, rj.y, rj.z, p.box, p.half, dx, dy, dz);
             if (r2 <= 0) continue;
             if ((r2 >= hi2) && (r2 >= hjd * hjd)) continue;
             const T r = Real<T>::sqrt_(T(r2));
