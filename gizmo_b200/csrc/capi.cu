@@ -948,17 +948,11 @@ int sym_rows_from_density(gz_context *c)
     const int n = c->n;
     cudaStream_t s = c->stream;
     const size_t N = (size_t)std::max(n, 1);
-    if (ensure(c, c->s_acnt, sizeof(int) * N) || ensure(c, c->s_bcnt, sizeof(int) * N) ||
-        ensure(c, c->s_counts, sizeof(long long) * N))
-        return c->err;
-    GZ_CUDA(c, cudaMemsetAsync(c->s_bcnt.p, 0, sizeof(int) * N, s));
-    sym_split(n, ptr<double>(c->x), ptr<double>(c->y), ptr<double>(c->z), ptr<double>(c->h), c->prm.box_size,
-              ptr<long long>(c->d_beg), ptr<long long>(c->d_end), ptr<int>(c->d_nbr), ptr<int>(c->s_acnt),
-              ptr<int>(c->s_bcnt), s);
+    if (ensure(c, c->s_counts, sizeof(long long) * N)) return c->err;
     sym_counts(n, ptr<int>(c->s_acnt), ptr<int>(c->s_bcnt), ptr<long long>(c->s_counts), s);
-    c->launches += 2;
+    c->launches += 1;
     GZ_CUDA(c, cudaGetLastError());
-    c->dens_all = false;  // the density rows are compacted in place: consumed
+    c->dens_all = false;  // the split density rows are consumed
     long long total = 0;
     if (exclusive_scan_counts(c, n, c->s_counts, c->s_off, &total)) return c->err;
     if (total > (long long)INT32_MAX * 4) return fail(c, GZ_ERR_CAPACITY, "neighbour rows exceed capacity");
@@ -1363,9 +1357,11 @@ __global__ void k_g_tree_check(const TreeBuild *tb, GraphState *gs)
     if (tb->fail) gs->fail |= kGraphFailTree;
 }
 
-// the flow sums of the na targets of a density pass, at their converged lengths
-// (captured: not taken once the graph has failed)
-void flow_sums(gz_context *c, int na, bool captured, cudaStream_t s)
+// The flow sums of the na targets of a density pass, at their converged lengths;
+// with every particle a target (`all`) the rows are split for the symmetric rows on
+// the way. Captured: nothing once the graph has failed. (Not under
+// GZ_TIMER_DENSITY_SUMS, which counts the iteration's rows.)
+int flow_sums(gz_context *c, int na, bool all, bool captured, cudaStream_t s)
 {
     DensityWork w{};
     w.gs = captured ? ptr<GraphState>(c->gstate) : nullptr;
@@ -1376,8 +1372,15 @@ void flow_sums(gz_context *c, int na, bool captured, cudaStream_t s)
     w.nbr = ptr<int>(c->d_nbr);
     w.rec = ptr<DensRec>(c->rec);
     w.acc = ptr<double>(c->acc);
-    // (not under GZ_TIMER_DENSITY_SUMS, which counts the iteration's rows)
-    density_sums(c->pp, view(c), w, DensitySums::flow, density_lanes(c, na), s);
+    if (!all) {
+        density_sums(c->pp, view(c), w, DensitySums::flow, density_lanes(c, na), s);
+        return 0;
+    }
+    if (ensure(c, c->s_acnt, sizeof(int) * (size_t)na) || ensure(c, c->s_bcnt, sizeof(int) * (size_t)na)) return c->err;
+    GZ_CUDA(c, cudaMemsetAsync(c->s_bcnt.p, 0, sizeof(int) * (size_t)na, s));
+    density_flow_split(c->pp, view(c), w, ptr<int>(c->d_nbr), ptr<int>(c->s_acnt), ptr<int>(c->s_bcnt),
+                       std::max(8, density_lanes(c, na)), s);
+    return 0;
 }
 
 int density_caps(const gz_context *c, int *cap0, int *cap1)
@@ -1597,10 +1600,6 @@ int capture_sym_rows(gz_context *c, cudaStream_t s, long long sym_cap, cudaGraph
 {
     const int n = c->n;
     const size_t N = (size_t)std::max(n, 1);
-    GZ_CUDA(c, cudaMemsetAsync(c->s_bcnt.p, 0, sizeof(int) * N, s));
-    sym_split(n, ptr<double>(c->x), ptr<double>(c->y), ptr<double>(c->z), ptr<double>(c->h), c->prm.box_size,
-              ptr<long long>(c->d_beg), ptr<long long>(c->d_end), ptr<int>(c->d_nbr), ptr<int>(c->s_acnt),
-              ptr<int>(c->s_bcnt), s);
     sym_counts(n, ptr<int>(c->s_acnt), ptr<int>(c->s_bcnt), ptr<long long>(c->s_counts), s);
     GZ_CUDA(c, cudaMemsetAsync(c->s_off.p, 0, sizeof(long long), s));
     size_t tmp = c->cub_tmp.bytes;
@@ -1699,7 +1698,7 @@ int graph_capture(gz_context *c, long long sym_cap, long long rq_cap, bool with_
         if ((rc = add_conditional(c, s, h_loop, cudaGraphCondTypeWhile, &body_loop))) break;
         if ((rc = body(s1, body_loop, [&] { return capture_density_iteration(c, s1, h_loop); }))) break;
         if ((rc = check_last(c, "density iteration"))) break;
-        flow_sums(c, n, true, s);
+        if ((rc = flow_sums(c, n, true, true, s))) break;
         density_finalize(c->pp, ps, ptr<double>(c->acc), ptr<int>(c->targets), n, s);
         if ((rc = make_handle(c, s, &h_conv, 0))) break;
         k_g_if_converged<<<1, 1, 0, s>>>(ptr<GraphState>(c->gstate), h_conv);
@@ -1730,12 +1729,12 @@ int graph_capture(gz_context *c, long long sym_cap, long long rq_cap, bool with_
     // setup (targets, active flags, prep, pack, state) + flow sums + finalize + the
     // convergence test; per iteration prep, radii, two walk modes, padded
     // rows, overflow check, overflow walk, three sums instances, after_iter,
-    // the selection's three steps, next; the rows' split, counts and check;
+    // the selection's three steps, next; the rows' counts and check;
     // scatter, sort, the gradient pack and rows, the force preloop, pack,
     // pairs, deferred pairs, (refine,) gather, finish
     c->g.kernels_top = 8 + restage_kernels;
     c->g.kernels_loop = 15;
-    c->g.kernels_sym = 3;
+    c->g.kernels_sym = 2;
     c->g.kernels_tail = c->prm.precision == GZ_PRECISION_MIXED ? 11 : 10;
     const cudaError_t ie = cudaGraphInstantiate(&c->g.exec, g, 0);
     if (ie != cudaSuccess) {
@@ -2200,7 +2199,7 @@ int gz_hydro_density(gz_context *c, const int *active, int n_active)
     }
     c->last_iters = iter;
     c->d_used = base;
-    flow_sums(c, na, false, s);
+    if (flow_sums(c, na, active == nullptr, false, s)) return c->err;
     c->launches++;
     density_finalize(c->pp, ps, ptr<double>(c->acc), ptr<int>(c->targets), na, s);
     if (na > 0) c->launches++;

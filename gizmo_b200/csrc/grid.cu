@@ -682,58 +682,10 @@ __global__ void __launch_bounds__(256) k_walk_graph_over(Tree t, const double *_
 
 // ------------------------------------------------ symmetric rows from density rows
 // When the density pass covered every particle, each particle's density row
-// holds every j with r < (row radius) >= its converged h, so the symmetric
-// rows follow without another tree walk:
-//   S_i = A_i u B_i,  A_i = {j : 0 < r2 < h_i^2},  B_i = {j : i in A_j, r2 >= h_i^2}
-// (r2 is bitwise symmetric: the minimum image of -d is the negation of that of
-// d), which is exactly the walk's predicate 0 < r2 and !(r2 >= h_i^2 and
-// r2 >= h_j^2). The rows are sorted at the end, so they equal the walk's.
-
-// Compacts density row i in place to A_i (order kept), marks an entry whose
-// pair is one-sided (r2 >= h_j^2: i belongs in B_j) by storing ~j, and counts
-// |A_i| and |B_j|.
-// (eight 256-thread blocks per multiprocessor, at most 32 registers: the
-// split waits on its position gathers, and full occupancy hides more of
-// them; 25.8 vs 26.1 ms for the 256^3 gradients stage at six blocks)
-template <int TPT>
-__global__ void __launch_bounds__(256, 8) k_sym_split(int n, const double *__restrict__ x, const double *__restrict__ y,
-                                                   const double *__restrict__ z, const double *__restrict__ h,
-                                                   double box, const long long *__restrict__ beg,
-                                                   const long long *__restrict__ end, int *nbr, int *acnt, int *bcnt)
-{
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = gtid / TPT, lane = gtid % TPT;
-    if (i >= n) return;
-    const int gshift = (threadIdx.x & 31) & ~(TPT - 1);
-    const unsigned mask = (TPT == 32) ? 0xffffffffu : (((1u << TPT) - 1u) << gshift);
-    const double half = 0.5 * box;
-    const double xi = x[i], yi = y[i], zi = z[i], hi = h[i];
-    const double hi2 = __dmul_rn(hi, hi);
-    const long long b0 = beg[i], b1 = end[i];
-    long long wpos = b0;
-    for (long long e0 = b0; e0 < b1; e0 += TPT) {
-        const long long e = e0 + lane;
-        int j = 0;
-        bool in_a = false, one_sided = false;
-        if (e < b1) {
-            j = nbr[e];
-            double dx, dy, dz;
-            const double r2 = sep2_near(xi, yi, zi, x[j], y[j], z[j], box, half, dx, dy, dz);
-            in_a = (r2 > 0) && (r2 < hi2);
-            if (in_a) {
-                const double hj = h[j];
-                one_sided = !(r2 < __dmul_rn(hj, hj));
-                if (one_sided) atomicAdd(bcnt + j, 1);
-            }
-        }
-        const unsigned gb = (__ballot_sync(mask, in_a) >> gshift) & (TPT == 32 ? 0xffffffffu : ((1u << TPT) - 1u));
-        __syncwarp(mask);  // every lane has read its entry before any is overwritten
-        if (in_a) nbr[wpos + __popc(gb & ((1u << lane) - 1u))] = one_sided ? ~j : j;
-        wpos += __popc(gb);
-    }
-    if (lane == 0) acnt[i] = (int)(wpos - b0);
-}
-
+// holds every j with r < (row radius) >= its converged h, so the symmetric rows
+// S_i = A_i u B_i follow without another tree walk: k_density_flow_split has
+// compacted the rows to A_i, marked the one-sided entries and counted. The rows
+// are sorted at the end, so they equal the walk's.
 __global__ void k_sym_counts(int n, const int *__restrict__ acnt, const int *__restrict__ bcnt, long long *cnt)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -800,12 +752,6 @@ __global__ void __launch_bounds__(256) k_sym_sort(int n, const long long *__rest
         }
         out[b0 + rank] = v;
     }
-}
-
-void sym_split(int n, const double *x, const double *y, const double *z, const double *h, double box,
-               const long long *beg, const long long *end, int *nbr, int *acnt, int *bcnt, cudaStream_t s)
-{
-    if (n > 0) k_sym_split<8><<<(unsigned)(((long long)n * 8 + 255) / 256), 256, 0, s>>>(n, x, y, z, h, box, beg, end, nbr, acnt, bcnt);
 }
 
 void sym_counts(int n, const int *acnt, const int *bcnt, long long *cnt, cudaStream_t s)

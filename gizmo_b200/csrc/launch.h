@@ -70,9 +70,7 @@ void long_rows(int rows, const int *t, const long long *counts, const long long 
 void copy_rows(int rows, const long long *counts, const long long *off, int cap, const int *padded, int *nbr,
                cudaStream_t s);
 
-// symmetric rows derived from the density rows of a pass over all particles
-void sym_split(int n, const double *x, const double *y, const double *z, const double *h, double box,
-               const long long *beg, const long long *end, int *nbr, int *acnt, int *bcnt, cudaStream_t s);
+// symmetric rows derived from the density rows of a pass over all particles (after density_flow_split)
 void sym_counts(int n, const int *acnt, const int *bcnt, long long *cnt, cudaStream_t s);
 void sym_scatter(int n, const long long *beg, const int *nbr, const int *acnt, const long long *s_off, int *bcur,
                  int *rows, cudaStream_t s);
@@ -107,6 +105,9 @@ void density_pack(const Particles &ps, DensRec *rec, cudaStream_t s);
 enum class DensitySums { all, shape, flow };
 void density_sums(const PassParams &p, const Particles &ps, const DensityWork &w, DensitySums what, int tpt,
                   cudaStream_t s);
+// the flow sums of every particle and the split of its density row (nbr, in place) for the symmetric rows
+void density_flow_split(const PassParams &p, const Particles &ps, const DensityWork &w, int *nbr, int *acnt, int *bcnt,
+                        int tpt, cudaStream_t s);
 void density_after_iter(const PassParams &p, const Particles &ps, const DensityWork &w, DevStatus *st, cudaStream_t s);
 // Captured-pass forms (GraphState): every TPT instance is launched with `blocks`
 // blocks and the one the device state names runs; after_iter writes the

@@ -78,37 +78,34 @@ template <int WHAT> GZ_DEV DensRec load_dens_rec(const DensRec *__restrict__ rec
     return r;
 }
 
-// The sums of target t's density row, by the TPT lanes (`lane` of them, on
-// `mask`) that own it; lane 0 stores them.
-template <typename T, int TPT, int WHAT>
-GZ_DEV void density_row(const PassParams &p, const Particles &ps, const DensityWork &w, int t, int lane,
-                        unsigned mask)
-{
-    constexpr bool kShape = WHAT != kSumsFlow, kFlow = WHAT != kSumsShape;
-    const double xi = ps.x[t], yi = ps.y[t], zi = ps.z[t];
-    const double hd = ps.h[t];
-    const double h2 = hd * hd;
-    const T h = T(hd);
-    T hinv, hinv3, hinv4;
-    k_hinv(h, hinv, hinv3, hinv4);
-    T vix = T(0), viy = T(0), viz = T(0);
-    if (kFlow) { vix = T(ps.vx[t]); viy = T(ps.vy[t]); viz = T(ps.vz[t]); }
-    const int mfv = p.method == 1;
+// A target of the density sums and the sums that are taken for it.
+template <typename T, int WHAT> struct DensityTarget {
+    static constexpr bool kShape = WHAT != kSumsFlow, kFlow = WHAT != kSumsShape;
+    double xi, yi, zi, h2;
+    T hinv, hinv3, hinv4, vix, viy, viz;
     double a[17];
+
+    GZ_DEV DensityTarget(const Particles &ps, int t)
+    {
+        xi = ps.x[t]; yi = ps.y[t]; zi = ps.z[t];
+        const double hd = ps.h[t];
+        h2 = hd * hd;
+        k_hinv(T(hd), hinv, hinv3, hinv4);
+        vix = viy = viz = T(0);
+        if (kFlow) { vix = T(ps.vx[t]); viy = T(ps.vy[t]); viz = T(ps.vz[t]); }
 #pragma unroll
-    for (int k = 0; k < 17; k++) a[k] = 0;
-    // one neighbour's contribution; the lane visits its entries in row order
-    auto pair = [&](const DensRec &rj) {
-        const double mjd = rj.m;
-        if (mjd <= 0) return;
-        double dx, dy, dz;
-        const double r2 = sep2_near(xi, yi, zi, rj.x, rj.y, rj.z, p.box, p.half, dx, dy, dz);
-        if (r2 >= h2) return;
+        for (int k = 0; k < 17; k++) a[k] = 0;
+    }
+
+    // one neighbour's contribution, at separation (dx, dy, dz) and its exact square
+    GZ_DEV void add(const PassParams &p, const DensRec &rj, double dx, double dy, double dz, double r2)
+    {
+        const int mfv = p.method == 1;
         const T r = Real<T>::sqrt_(T(r2));
         const T u = r * hinv;
         T wk, dwk;
         k_main(p.kernel, u, hinv3, hinv4, wk, dwk);
-        const T mj_wk = T(mjd) * wk;
+        const T mj_wk = T(rj.m) * wk;
         const T vjx = T(rj.vx), vjy = T(rj.vy), vjz = T(rj.vz);
         if (kShape) a[0] += (double)wk;
         if (kFlow) {
@@ -143,7 +140,29 @@ GZ_DEV void density_row(const PassParams &p, const Particles &ps, const DensityW
                 a[3] -= (double)(dwk * (px * dvx + py * dvy + pz * dvz) / r);
             }
         }
-    };
+    }
+
+    // summed over the row's TPT lanes; lane 0 stores them
+    template <int TPT> GZ_DEV void store(const DensityWork &w, int n_particles, int t, int lane, unsigned mask)
+    {
+        const size_t n = (size_t)n_particles;
+#pragma unroll
+        for (int k = 0; k < 17; k++) {
+            const bool flow = k == 1 || k == 3 || k >= 14;
+            if (k == 13 || (flow ? !kFlow : !kShape)) continue;
+            a[k] = warp_sum(a[k], mask, TPT);
+            if (lane == 0) w.acc[k * n + t] = a[k];
+        }
+    }
+};
+
+// The sums of target t's density row, by the TPT lanes (`lane` of them, on
+// `mask`) that own it; each visits its entries in row order.
+template <typename T, int TPT, int WHAT>
+GZ_DEV void density_row(const PassParams &p, const Particles &ps, const DensityWork &w, int t, int lane,
+                        unsigned mask)
+{
+    DensityTarget<T, WHAT> me(ps, t);
     // one record in flight per lane: the register budget goes to resident
     // warps (kDensityBlocks of 128 threads per multiprocessor), which hide the
     // gather latency better than a second record per lane does; the next
@@ -156,17 +175,14 @@ GZ_DEV void density_row(const PassParams &p, const Particles &ps, const DensityW
     for (; e < b1; e += TPT) {
         const long long en = e + TPT;
         const int jn = en < b1 ? __ldg(nbr + en) : 0;
-        pair(load_dens_rec<WHAT>(w.rec, j));
+        const DensRec rj = load_dens_rec<WHAT>(w.rec, j);
         j = jn;
+        if (rj.m <= 0) continue;
+        double dx, dy, dz;
+        const double r2 = sep2_near(me.xi, me.yi, me.zi, rj.x, rj.y, rj.z, p.box, p.half, dx, dy, dz);
+        if (!(r2 >= me.h2)) me.add(p, rj, dx, dy, dz, r2);
     }
-    const size_t n = (size_t)ps.n;
-#pragma unroll
-    for (int k = 0; k < 17; k++) {
-        const bool flow = k == 1 || k == 3 || k >= 14;
-        if (k == 13 || (flow ? !kFlow : !kShape)) continue;
-        a[k] = warp_sum(a[k], mask, TPT);
-        if (lane == 0) w.acc[k * n + t] = a[k];
-    }
+    me.template store<TPT>(w, ps.n, t, lane, mask);
 }
 
 // Resident 128-thread blocks per multiprocessor the density sums ask of the
@@ -214,6 +230,58 @@ __global__ void __launch_bounds__(kDensityBlock, kDensityBlocks<kSumsShape>)
         const int slot = chunk * kRows + (int)threadIdx.x / TPT;
         if (slot < n_todo) density_row<T, TPT, kSumsShape>(p, ps, w, todo[slot], lane, mask);
     }
+}
+
+// The flow sums of a pass over every particle, and on the way the first step of the
+// symmetric rows, which reads the same neighbours. With A_i = {j : 0 < r2 < h_i^2},
+// the symmetric row is S_i = A_i u B_i, B_i = {j : i in A_j, r2 >= h_i^2} (r2 is
+// bitwise symmetric: the minimum image of -d is the negation of that of d), which is
+// exactly the walk's predicate 0 < r2 and !(r2 >= h_i^2 and r2 >= h_j^2). This
+// compacts density row i in place to A_i (order kept), stores ~j for an entry whose
+// pair is one-sided (r2 >= h_j^2: i belongs in B_j), and counts |A_i| and |B_j|.
+// The flow sums and a split of their own took, density and gradient stages together,
+// 19.6 / 19.6 / 12.7 ms for 2M lognormal, 2M Plummer and a million Plummer particles
+// (FP64) and 2.72 ms for 110,003 lognormal ones; this takes 19.5 / 19.3 / 12.4 /
+// 2.68 ms at eight lanes a row at least (four: 19.9 / 19.6 / 12.7) and eight blocks
+// per multiprocessor (seven 19.7 / 19.4 / 12.4, six 20.3 / 19.9 / 12.9 at four lanes).
+template <typename T, int TPT>
+__global__ void __launch_bounds__(kDensityBlock, kDensityBlocks<kSumsFlow>) k_density_flow_split(PassParams p, Particles ps,
+                                                                                                DensityWork w, int *nbr,
+                                                                                                int *acnt, int *bcnt)
+{
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = gtid / TPT, lane = gtid % TPT;
+    if (t >= w.n_todo || (w.gs && w.gs->fail)) return;  // (every particle is a target: slot t holds t)
+    const int gshift = (threadIdx.x & 31) & ~(TPT - 1);
+    const unsigned group = (1u << TPT) - 1u, mask = group << gshift;
+    DensityTarget<T, kSumsFlow> me(ps, t);
+    const long long b0 = w.beg[t], b1 = w.end[t];
+    long long wpos = b0;
+    int jn = b0 + lane < b1 ? nbr[b0 + lane] : 0;
+    for (long long e0 = b0; e0 < b1; e0 += TPT) {
+        const int j = jn;
+        // (the next entries are read before any place past them is written)
+        jn = e0 + TPT + lane < b1 ? nbr[e0 + TPT + lane] : 0;
+        bool in_a = false, one_sided = false;
+        if (e0 + lane < b1) {
+            const DensRec rj = load_dens_rec<kSumsFlow>(w.rec, j);
+            double dx, dy, dz;
+            const double r2 = sep2_near(me.xi, me.yi, me.zi, rj.x, rj.y, rj.z, p.box, p.half, dx, dy, dz);
+            in_a = r2 > 0 && r2 < me.h2;
+            if (in_a) {
+                const double hj = ps.h[j];
+                one_sided = !(r2 < __dmul_rn(hj, hj));
+                if (one_sided) atomicAdd(bcnt + j, 1);
+            }
+            if (!(rj.m <= 0) && !(r2 >= me.h2)) me.add(p, rj, dx, dy, dz, r2);
+        }
+        const unsigned gb = (__ballot_sync(mask, in_a) >> gshift) & group;
+        __syncwarp(mask);  // every lane has read its entry before any is overwritten
+        if (in_a) nbr[wpos + __popc(gb & ((1u << lane) - 1u))] = one_sided ? ~j : j;
+        wpos += __popc(gb);
+    }
+    if (lane == 0) acnt[t] = (int)(wpos - b0);
+    me.template store<TPT>(w, ps.n, t, lane, mask);
 }
 
 template <typename T, int WHAT>
@@ -374,11 +442,9 @@ void launch_gradients(const PassParams &p, const Particles &ps, const int *targe
     const unsigned blocks = (unsigned)((threads + 127) / 128);  // 128-thread blocks: finer register granularity
     if (ev) cudaEventRecord(ev->start, s);
     switch (tpt) {
-        case 1: k_gradients<T, 1><<<blocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, rec); break;
         case 2: k_gradients<T, 2><<<blocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, rec); break;
         case 4: k_gradients<T, 4><<<blocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, rec); break;
         case 8: k_gradients<T, 8><<<blocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, rec); break;
-        case 32: k_gradients<T, 32><<<blocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, rec); break;
         default: k_gradients<T, 16><<<blocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, rec); break;
     }
     if (ev) cudaEventRecord(ev->stop, s);

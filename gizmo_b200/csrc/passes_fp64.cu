@@ -47,6 +47,18 @@ void density_sums(const PassParams &p, const Particles &ps, const DensityWork &w
     }
 }
 
+void density_flow_split(const PassParams &p, const Particles &ps, const DensityWork &w, int *nbr, int *acnt, int *bcnt,
+                        int tpt, cudaStream_t s)
+{
+    if (w.n_todo <= 0) return;
+    const unsigned blocks = (unsigned)(((long long)w.n_todo * tpt + kDensityBlock - 1) / kDensityBlock);
+    switch (tpt) {
+        case 4: k_density_flow_split<double, 4><<<blocks, kDensityBlock, 0, s>>>(p, ps, w, nbr, acnt, bcnt); break;
+        case 8: k_density_flow_split<double, 8><<<blocks, kDensityBlock, 0, s>>>(p, ps, w, nbr, acnt, bcnt); break;
+        default: k_density_flow_split<double, 16><<<blocks, kDensityBlock, 0, s>>>(p, ps, w, nbr, acnt, bcnt); break;
+    }
+}
+
 void density_sums_graph(const PassParams &p, const Particles &ps, const DensityWork &w, GraphState *gs,
                         const int *todo, int blocks, cudaStream_t s)
 {
