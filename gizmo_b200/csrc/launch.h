@@ -96,10 +96,6 @@ struct DensityWork {
 };
 
 // passes_fp64.cu / passes_mixed.cu (same kernels, pair arithmetic double / float)
-struct PassLaunch {
-    int tpt_density, tpt_gradient, tpt_force;
-};
-
 void density_pack(const Particles &ps, DensRec *rec, cudaStream_t s);
 // the sums of w.todo's rows: all 17, the ones the iteration decides on, or the others
 enum class DensitySums { all, shape, flow };
@@ -131,10 +127,10 @@ void gradients_fp64(const PassParams &p, const Particles &ps, const int *targets
 // `all`: every particle is a target (flux then holds each pair once). The
 // mixed form needs flux; q receives its fragile pairs (cap >= 1), dq the pairs
 // deferred to their own kernel (cap >= 1 with flux; its count zeroed by the caller).
-void force_fp64(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
+void force_fp64(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows,
                 DevStatus *st, void *rec, void *flux, bool all, const RefineQueue &dq, double *sums,
                 const EventPair *ev, cudaStream_t s);
-void force_mixed(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
+void force_mixed(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows,
                  DevStatus *st, void *rec, void *flux, bool all, const RefineQueue &q, const RefineQueue &dq,
                  double *sums, const EventPair *ev, cudaStream_t s);
 // The queued pairs of a mixed-form pass evaluated in FP64 from the FP64 mirror

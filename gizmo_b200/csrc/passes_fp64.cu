@@ -73,12 +73,12 @@ void gradients_fp64(const PassParams &p, const Particles &ps, const int *targets
     launch_gradients<double>(p, ps, targets, n_targets, rows, tpt, rec, ev, s);
 }
 
-void force_fp64(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
+void force_fp64(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows,
                 DevStatus *st, void *rec, void *flux, bool all, const RefineQueue &dq, double *sums,
                 const EventPair *ev, cudaStream_t s)
 {
     const RefineQueue none{nullptr, nullptr, 0};
-    launch_force<double>(p, ps, targets, n_targets, rows, tpt, st, rec, flux, all, none, dq, sums, ev, s);
+    launch_force<double>(p, ps, targets, n_targets, rows, st, rec, flux, all, none, dq, sums, ev, s);
 }
 
 // force_refine: one thread per queued pair, grid-stride over the count the

@@ -7,11 +7,11 @@
 
 namespace gz {
 
-void force_mixed(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
+void force_mixed(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows,
                  DevStatus *st, void *rec, void *flux, bool all, const RefineQueue &q, const RefineQueue &dq,
                  double *sums, const EventPair *ev, cudaStream_t s)
 {
-    launch_force<float>(p, ps, targets, n_targets, rows, tpt, st, rec, flux, all, q, dq, sums, ev, s);
+    launch_force<float>(p, ps, targets, n_targets, rows, st, rec, flux, all, q, dq, sums, ev, s);
 }
 
 }  // namespace gz
