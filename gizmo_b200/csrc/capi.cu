@@ -919,12 +919,26 @@ int build_tree(gz_context *c)
                       c->box_bits ? ptr<int>(c->box_of) : nullptr, c->box_bits ? ptr<int>(c->root_of) : nullptr,
                       c->sms * 8, s);
     c->launches += tree_build_launches(n);
+    // the bottom-up pass of a small set is queued over the nodes held, before the node
+    // count is read back (the device does not idle meanwhile); a large one's waits for it
+    const bool small = n <= kGatherAllMax;
+    if (small) {
+        if (ensure(c, c->t_lo, sizeof(double4) * (size_t)cap) || ensure(c, c->t_hi, sizeof(double4) * (size_t)cap) ||
+            ensure(c, c->t_done, sizeof(int) * (size_t)cap))
+            return c->err;
+        tree_up((int)cap, ptr<int4>(c->t_node), ptr<int>(c->t_parent), ptr<double>(c->x), ptr<double>(c->y),
+                ptr<double>(c->z), ptr<double>(c->h), ptr<double4>(c->t_lo), ptr<double4>(c->t_hi), ptr<int>(c->t_done), 1,
+                s, &ptr<TreeBuild>(c->t_build)->total);
+        c->launches++;
+    }
     TreeBuild tb{};
     GZ_CUDA(c, cudaMemcpyAsync(&tb, c->t_build.p, sizeof(tb), cudaMemcpyDeviceToHost, s));
     GZ_CUDA(c, cudaStreamSynchronize(s));
     if (tb.fail) return build_tree_levels(c);
     c->t_nodes = tb.total;
     c->t_levels = tb.L;
+    GZ_CUDA(c, cudaGetLastError());
+    if (small) return 0;
     if (ensure(c, c->t_lo, sizeof(double4) * (size_t)c->t_nodes) || ensure(c, c->t_hi, sizeof(double4) * (size_t)c->t_nodes) ||
         ensure(c, c->t_done, sizeof(int) * (size_t)c->t_nodes))
         return c->err;
@@ -1587,7 +1601,7 @@ int capture_density_iteration(gz_context *c, cudaStream_t s, cudaGraphConditiona
     w.h_iter_max = ptr<unsigned long long>(c->hmax);
     w.keep = ptr<unsigned char>(c->keep);
     w.regrow = ptr<unsigned char>(c->regrow);
-    density_sums_graph(c->pp, ps, w, gs, ptr<int>(c->todo_a), c->sms * 6, s);
+    density_sums_graph(c->pp, ps, w, gs, ptr<int>(c->todo_a), c->sms * 8, s);
     density_after_iter_graph(c->pp, ps, w, ptr<DevStatus>(c->status), gs, ptr<int>(c->todo_a), c->sms * 16, s);
     int *ca = ptr<int>(c->g_sel), *cb = ca + (n + kSelChunk - 1) / kSelChunk;
     k_sel_count<<<c->sms * 2, kSelChunk, 0, s>>>(gs, ptr<unsigned char>(c->keep), ptr<unsigned char>(c->regrow), ca, cb);
@@ -1734,12 +1748,12 @@ int graph_capture(gz_context *c, long long sym_cap, long long rq_cap, bool with_
     // this library's kernels in each part (the key sort and scans are CUB's):
     // setup (targets, active flags, prep, pack, state) + flow sums + finalize + the
     // convergence test; per iteration prep, radii, two walk modes, padded
-    // rows, overflow check, overflow walk, three sums instances, after_iter,
+    // rows, overflow check, overflow walk, sums, after_iter,
     // the selection's three steps, next; the rows' counts and check;
     // scatter, sort, the gradient pack and rows, the force preloop, pack,
     // pairs, deferred pairs, (refine,) gather, finish
     c->g.kernels_top = 8 + restage_kernels;
-    c->g.kernels_loop = 15;
+    c->g.kernels_loop = 13;
     c->g.kernels_sym = 2;
     c->g.kernels_tail = c->prm.precision == GZ_PRECISION_MIXED ? 11 : 10;
     const cudaError_t ie = cudaGraphInstantiate(&c->g.exec, g, 0);

@@ -105,8 +105,8 @@ void density_sums(const PassParams &p, const Particles &ps, const DensityWork &w
 void density_flow_split(const PassParams &p, const Particles &ps, const DensityWork &w, int *nbr, int *acnt, int *bcnt,
                         int tpt, cudaStream_t s);
 void density_after_iter(const PassParams &p, const Particles &ps, const DensityWork &w, DevStatus *st, cudaStream_t s);
-// Captured-pass forms (GraphState): every TPT instance is launched with `blocks`
-// blocks and the one the device state names runs; after_iter writes the
+// Captured-pass forms (GraphState): `blocks` blocks take the iteration's rows with
+// the lanes the device state names; after_iter writes the
 // per-slot flags of w.keep and w.regrow for the iteration's target count.
 void density_sums_graph(const PassParams &p, const Particles &ps, const DensityWork &w, GraphState *gs,
                         const int *todo, int blocks, cudaStream_t s);

@@ -208,18 +208,16 @@ __global__ void __launch_bounds__(kDensityBlock, kDensityBlocks<WHAT>) k_density
 // plain launch's grid: each takes the next block-sized chunk of rows (the
 // plain grid's next block) from a counter, so the rows in flight are a
 // contiguous run of the list and the chunks go to whichever block is free, as
-// the hardware hands out the blocks of a plain launch. An instance whose TPT
-// is not the iteration's returns at once. Each row is summed by the same
-// lanes in the same order as k_density_sums sums it.
+// the hardware hands out the blocks of a plain launch. Each row is summed by the
+// same lanes in the same order as k_density_sums sums it. (One kernel for the three
+// lane counts: a launch of its own each cost the iteration two empty ones.)
 template <typename T, int TPT>
-__global__ void __launch_bounds__(kDensityBlock, kDensityBlocks<kSumsShape>)
-    k_density_sums_graph(PassParams p, Particles ps, DensityWork w, GraphState *gs, const int *__restrict__ todo)
+GZ_DEV void density_chunks(const PassParams &p, const Particles &ps, const DensityWork &w, GraphState *gs,
+                           const int *__restrict__ todo, int &s_chunk)
 {
-    __shared__ int s_chunk;
-    if (gs->fail || gs->tpt != TPT) return;
     const int n_todo = gs->n_todo;
     constexpr int kRows = kDensityBlock / TPT;
-    const unsigned mask = (TPT == 32) ? 0xffffffffu : (((1u << TPT) - 1u) << ((threadIdx.x & 31) & ~(TPT - 1)));
+    const unsigned mask = ((1u << TPT) - 1u) << ((threadIdx.x & 31) & ~(TPT - 1));
     const int lane = threadIdx.x % TPT;
     for (;;) {
         if (threadIdx.x == 0) s_chunk = atomicAdd(&gs->sums_next, 1);
@@ -229,6 +227,19 @@ __global__ void __launch_bounds__(kDensityBlock, kDensityBlocks<kSumsShape>)
         if ((long long)chunk * kRows >= n_todo) break;
         const int slot = chunk * kRows + (int)threadIdx.x / TPT;
         if (slot < n_todo) density_row<T, TPT, kSumsShape>(p, ps, w, todo[slot], lane, mask);
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kDensityBlock, kDensityBlocks<kSumsShape>)
+    k_density_sums_graph(PassParams p, Particles ps, DensityWork w, GraphState *gs, const int *__restrict__ todo)
+{
+    __shared__ int s_chunk;
+    if (gs->fail) return;
+    switch (gs->tpt) {
+        case 4: density_chunks<T, 4>(p, ps, w, gs, todo, s_chunk); break;
+        case 8: density_chunks<T, 8>(p, ps, w, gs, todo, s_chunk); break;
+        default: density_chunks<T, 16>(p, ps, w, gs, todo, s_chunk); break;
     }
 }
 

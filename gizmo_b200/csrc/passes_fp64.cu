@@ -62,9 +62,7 @@ void density_flow_split(const PassParams &p, const Particles &ps, const DensityW
 void density_sums_graph(const PassParams &p, const Particles &ps, const DensityWork &w, GraphState *gs,
                         const int *todo, int blocks, cudaStream_t s)
 {
-    k_density_sums_graph<double, 4><<<blocks, kDensityBlock, 0, s>>>(p, ps, w, gs, todo);
-    k_density_sums_graph<double, 8><<<blocks, kDensityBlock, 0, s>>>(p, ps, w, gs, todo);
-    k_density_sums_graph<double, 16><<<blocks, kDensityBlock, 0, s>>>(p, ps, w, gs, todo);
+    k_density_sums_graph<double><<<blocks, kDensityBlock, 0, s>>>(p, ps, w, gs, todo);
 }
 
 void gradients_fp64(const PassParams &p, const Particles &ps, const int *targets, int n_targets, Csr rows, int tpt,
