@@ -222,32 +222,37 @@ int fail(gz_context *c, int code, const char *what)
 
 template <typename T> T *ptr(DevBuf &b) { return (T *)b.p; }
 
-int ensure(gz_context *c, DevBuf &b, size_t bytes)
-{
-    if (b.bytes >= bytes && b.p) return 0;
-    if (b.p) cudaFree(b.p);
-    b.p = nullptr;
-    b.bytes = 0;
-    size_t want = bytes > 0 ? bytes : 16;
-    GZ_CUDA(c, cudaMalloc(&b.p, want));
-    b.bytes = want;
-    return 0;
-}
-
-// like ensure(), but a failed allocation is not an error of the context
+// The buffer at `bytes` or more; false when it cannot be had (the error is cleared).
+// A buffer that has to grow grows by a quarter more than asked: the row totals of an
+// evolving set creep up from step to step, and freeing and allocating the row and
+// flux buffers in each of them cost 2 to 9 ms of a 2 ms step of 64,000 cells.
 bool try_ensure(DevBuf &b, size_t bytes)
 {
     if (b.bytes >= bytes && b.p) return true;
+    const size_t exact = bytes > 0 ? bytes : 16;
+    size_t want = b.p ? exact + exact / 4 : exact;
     if (b.p) cudaFree(b.p);
     b.p = nullptr;
     b.bytes = 0;
-    if (cudaMalloc(&b.p, bytes > 0 ? bytes : 16) != cudaSuccess) {
+    if (cudaMalloc(&b.p, want) != cudaSuccess) {
         cudaGetLastError();  // clear the allocation failure
         b.p = nullptr;
-        return false;
+        want = exact;
+        if (cudaMalloc(&b.p, want) != cudaSuccess) {
+            cudaGetLastError();
+            b.p = nullptr;
+            return false;
+        }
     }
-    b.bytes = bytes > 0 ? bytes : 16;
+    b.bytes = want;
     return true;
+}
+
+// like try_ensure(), and a failed allocation is an error of the context
+int ensure(gz_context *c, DevBuf &b, size_t bytes)
+{
+    if (!try_ensure(b, bytes)) return fail(c, GZ_ERR_CUDA, "out of device memory");
+    return 0;
 }
 
 void release(DevBuf &b)
