@@ -39,17 +39,18 @@ UNIT = "particle-updates/s"
 
 # per-pair FLOP constants (FMA = 2, sqrt/div/exp/log = 1 each), counted by hand
 # over the taken MFV ideal-gas branch of the pair bodies (HLLC solved on the
-# first try). Density, per accepted pair: separation 8, sqrt 1, u 1, cubic
-# kernel and derivative 10, the 17 sums 52 -> 72. Gradient ~60, force ~430.
-FLOPS_PER_PAIR = {"density": 72.0, "gradients": 60.0, "force": 430.0}
+# first try). Density, per accepted pair of the iteration's shape sums: separation
+# 8, sqrt 1, u 1, cubic kernel and derivative 10, the 11 sums 29 -> 49 (the flow
+# sums follow once, outside the timer). Gradient ~60, force ~430.
+FLOPS_PER_PAIR = {"density": 49.0, "gradients": 60.0, "force": 430.0}
 
 # DRAM bytes per work unit of a kernel from one ncu capture of the 64^3 case
 # (dram__bytes_read.sum + dram__bytes_write.sum over the units of the captured
 # launch), scaled to the units of a launch here: density sums per row
-# (profiles/density_sums_plummer64.md: 140.1 MB over 262,144 rows), the force
+# (profiles/density_sums_plummer64.md: 102.9 MB over 262,144 rows), the force
 # pair kernel per pair (profiles/force_pairs_plummer64.md: 1313.8 MB over
 # 7,841,073 pairs).
-DRAM_BYTES_PER_UNIT = {"density_sums": 140.1e6 / 262144, "force": 1313.8e6 / 7841073}
+DRAM_BYTES_PER_UNIT = {"density_sums": 102.9e6 / 262144, "force": 1313.8e6 / 7841073}
 
 
 def parse_args():
@@ -465,7 +466,7 @@ def run_ours(args, world, rank, local):
             e["traffic_bytes_per_launch"] = DRAM_BYTES_PER_UNIT[name] * e["units_per_launch"]
         kernels[name] = e
     dom = max((k for k in kernels if "achieved" in kernels[k]), key=lambda k: kernels[k]["ms_per_step"], default=None)
-    kernel_names = {"density_sums": "k_density_sums<double> (FP64 density sums, all h iterations)",
+    kernel_names = {"density_sums": "k_density_sums<double> (FP64 shape sums of the density rows, all h iterations)",
                     "force": "k_force_pairs<float> (MFV pair flux, each pair once)",
                     "gradients": "k_gradients<double> (least-squares gradients, FP64 in both forms)"}
     roofline = None

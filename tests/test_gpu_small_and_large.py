@@ -1,0 +1,74 @@
+"""Edges of the size rules of the restage and the download: the octree's narrow levels by one cluster and its wide
+ones by launches, with trees deeper than the levels that have a launch; box sets with empty boxes; and the
+fields' way back to the caller's order on both sides of the size from which scalars are gathered."""
+import numpy as np
+import pytest
+
+from gizmo_b200 import ics
+from gizmo_b200.hydro import HydroPass
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _nested(n, rng):
+    """Clumps inside clumps down to 2^-18 of the box, and 40 coincident particles: leaves at every level."""
+    scale = 2.0 ** -rng.integers(0, 19, n)
+    pos = (np.array([0.3, 0.6, 0.2]) + (rng.random((n, 3)) - 0.5) * scale[:, None]) % 1.0
+    pos[:min(n, 40)] = pos[0]
+    return pos
+
+
+@pytest.mark.parametrize("n", [1, 96, 97, 3000, 65536, 65537, 150000])
+def test_rows_of_deep_trees(n):
+    rng = np.random.default_rng(n)
+    wl = ics.sedov(4)
+    pos = _nested(n, rng)
+    # kernels of about twice the clump a particle lies in, shortened where the clump is crowded
+    r = np.abs((pos - np.array([0.3, 0.6, 0.2]) + 0.5) % 1.0 - 0.5).max(1)
+    h = np.clip(1.5 * r * (300.0 / max(n, 300)) ** (1 / 3), 1e-7, 0.2)
+    z = np.zeros((n, 3))
+    with HydroPass(wl.params) as hp:
+        hp.upload(pos, z, np.full(n, 1.0 / n), np.ones(n), np.full(n, 2.0 ** -8), h)
+        off, nbr = hp.neighbors(0)
+    st = O.new_state(n, dict(pos=pos, vel=z, mass=np.full(n, 1.0 / n), u=np.ones(n), dt=np.full(n, 2.0 ** -8), h=h))
+    ooff, onbr = O.neighbors(wl.params, st, 0)
+    assert np.array_equal(off, ooff) and np.array_equal(nbr, onbr)
+
+
+def test_box_sets_with_empty_boxes():
+    a, b = ics.shock_tube(8, seed=5), ics.sedov(9, seed=6)
+    counts = [0, a.n, 0, 0, b.n, 0]
+    cat = {k: np.concatenate([getattr(a, k), getattr(b, k)]) for k in ("pos", "vel", "mass", "u", "dt", "h")}
+    alone = []
+    for wl in (a, b):
+        with HydroPass(wl.params) as hp:
+            hp.upload_workload(wl)
+            alone.append(hp.neighbors(0))
+    with HydroPass(a.params) as hp:
+        hp.set_boxes(counts)
+        hp.upload(**cat)
+        off, nbr = hp.neighbors(0)
+    (oa, na), (ob, nb) = alone
+    assert np.array_equal(off, np.concatenate([oa, oa[-1] + ob[1:]]))
+    assert np.array_equal(nbr, np.concatenate([na, nb + a.n]))
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 87381, (1 << 18) + 1, (1 << 20) - 1, 1 << 20])
+def test_fields_return_in_the_callers_order(n):
+    import torch
+
+    rng = np.random.default_rng(n)
+    pos, h, cond = rng.random((n, 3)), rng.uniform(1e-3, 2e-3, n), rng.random(n)
+    wl = ics.sedov(4)
+    names = ["h", "cond", "rho", "nvt", "grad_v", "accel", "iters"]
+    with HydroPass(wl.params) as hp:
+        hp.upload(pos, np.zeros((n, 3)), np.ones(n), np.ones(n), np.full(n, 2.0 ** -8), h, cond)
+        out = hp.download(names)
+        pinned = {k: torch.empty(n, dtype=torch.float64, pin_memory=True) for k in ("h", "cond")}
+        hp.download_raw_async({k: v.data_ptr() for k, v in pinned.items()})
+        hp.wait()
+    assert np.array_equal(out["h"], h) and np.array_equal(out["cond"], cond)
+    assert np.array_equal(pinned["h"].numpy(), h) and np.array_equal(pinned["cond"].numpy(), cond)
+    for k in names[2:]:
+        assert not out[k].any(), k
