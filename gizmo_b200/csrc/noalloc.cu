@@ -7,7 +7,7 @@
 // gz_context, which allocates its buffers. This entry point computes the same
 // fixed-h density sums as gz_density_sums for a particle set that the caller
 // already holds in device memory, and allocates nothing: its only scratch is
-// the static Scratch below (3.2 MiB of device memory) that every GPU loading this
+// the static Scratch below (2.1 MiB of device memory) that every GPU loading this
 // library holds until the process exits.
 //
 // The particles are put in Morton order first, so that runs of 32 have small
@@ -17,7 +17,7 @@
 // inside the support take the exact FP64 test and the sums, whose arithmetic is
 // the one of k_density_sums in FP64 (this file is built with -fmad=false like
 // passes_fp64.cu), so the sums agree with gz_density_sums up to summation order.
-#include <cub/cub.cuh>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -35,9 +35,10 @@ constexpr int kSlices = 8;    // warps of a block, each taking its share of the 
 constexpr int kShare = kRun / kSlices;  // candidates a warp takes from each run
 constexpr int kHits = 32;     // screened candidates a lane holds before the warp evaluates them
 constexpr int kFewHits = 8;   // up to as many of a target are evaluated by its own lane
-constexpr int kKeyBits = 24;  // Morton key, 8 bits an axis: three 8-bit radix passes
+constexpr int kDigits = 256;  // Morton key, 8 bits an axis: three 8-bit radix passes
+constexpr int kSortBlocks = 8, kSortWarps = 32;  // the cluster that sorts
+constexpr int kSortRounds = kMaxParticles / (kSortBlocks * kSortWarps * 32);  // most particles a lane holds
 constexpr int kMaxDevices = 128;
-constexpr size_t kSortBytes = 1 << 20;
 static_assert(kMaxParticles <= 65536, "a hit is a 16-bit particle index");
 
 // Bounding box of a run, rounded outward to FP32: lo.w the largest coordinate
@@ -50,11 +51,11 @@ struct RunBox {
 // call reads it has written itself, so nothing in it needs clearing.
 struct Scratch {
     unsigned key[2][kMaxParticles];
-    int order[2][kMaxParticles];              // sorted -> caller's index: [1] after the sort
+    int order[2][kMaxParticles];              // sorted -> caller's index: [0] after the sort
     float4 pos[kMaxParticles];                // sorted FP32 positions; w: the caller's index
     RunBox box[kMaxParticles / kRun];
-    unsigned char sort[kSortBytes];           // temporary storage of the radix sort
 };
+static_assert(sizeof(Scratch) <= 2162688, "the documented size (2.1 MiB) is out of date");
 static __device__ __align__(256) Scratch g_scratch;
 
 std::mutex g_setup_mutex;
@@ -74,17 +75,126 @@ __device__ unsigned spread8(unsigned x)
     return (x | (x << 2)) & 0x249249u;
 }
 
-__global__ void k_noalloc_keys(int n, const double *__restrict__ pos, double box, unsigned *key, int *order)
+// Morton key of caller's particle i (the order only has to be good: coordinates outside the box are clamped)
+__device__ unsigned key_of(const double *__restrict__ pos, int i, double box)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     unsigned k = 0;
-    for (int c = 0; c < 3; c++) {  // (the order only has to be good: coordinates outside the box are clamped)
+    for (int c = 0; c < 3; c++) {
         const double v = pos[3 * (size_t)i + c] / box * 256.0;
         k |= spread8(v > 0.0 ? (v < 255.0 ? (unsigned)v : 255u) : 0u) << c;
     }
-    key[i] = k;
-    order[i] = i;
+    return k;
+}
+
+// The caller's particles in the order of their Morton keys, equal keys in the caller's order: a stable radix sort of
+// three 8-bit digits by one cluster. Each warp owns a run of consecutive places and holds its particles in registers
+// from their count to their scatter; the warps' counts become offsets in shared memory, the blocks' in distributed
+// shared memory, and the cluster's barrier separates the passes.
+//
+// The sort is this file's own, and one launch whatever n is, for what the entry point promises: a library's sort picks
+// its kernels by n, so that the first larger call loads new ones (which can need device memory and a synchronisation
+// when the caller has neither to give), and its blocks wait on flags in the scratch, which a second, overlapping call
+// rewrites. Here a place is computed from registers and shared memory alone and always lies in [0, n).
+// It is bound by the latency of its three passes' barriers and loads, on eight multiprocessors: whole call 29, 66, 105,
+// 171, 248 and 533 us at 100, 1,000, 4,000, 10,000, 20,000 and 65,536 particles, with a library's sort 27, 64, 103, 198,
+// 268 and 529.
+__global__ void __cluster_dims__(kSortBlocks, 1, 1) __launch_bounds__(32 * kSortWarps)
+    k_noalloc_sort(int n, const double *__restrict__ pos, double box, Scratch *g)
+{
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cluster = cg::this_cluster();
+    __shared__ unsigned short s_cnt[kSortWarps][kDigits];  // a warp's particles of each digit, then those of the warps before it
+    __shared__ int s_total[kDigits];                       // the block's particles of each digit
+    __shared__ int s_base[kDigits];                        // places before the block's particles of each digit
+    __shared__ int s_sum[kDigits / 32];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rank = (int)cluster.block_rank();
+    // places of a warp: a multiple of 32, the same for every warp
+    const int per = ((n + kSortBlocks * kSortWarps - 1) / (kSortBlocks * kSortWarps) + 31) / 32 * 32;
+    const int first = (rank * kSortWarps + warp) * per + lane;
+    for (int pass = 0; pass < 3; pass++) {
+        const int src = pass == 1 ? 0 : 1, dst = 1 - src;  // the keys' way: -> 0 -> 1 -> 0
+        unsigned key[kSortRounds];
+        int idx[kSortRounds];
+        unsigned short at[kSortRounds];  // place among the warp's particles of the digit
+#pragma unroll
+        for (int r = 0; r < kSortRounds; r++) {
+            const int e = first + 32 * r;
+            key[r] = 0;
+            idx[r] = e;
+            if (32 * r < per && e < n) {
+                if (pass == 0) {
+                    key[r] = key_of(pos, e, box);
+                } else {
+                    key[r] = __ldcg(&g->key[src][e]);
+                    idx[r] = __ldcg(&g->order[src][e]);
+                }
+            }
+        }
+        for (int k = threadIdx.x; k < kSortWarps * kDigits; k += 32 * kSortWarps) (&s_cnt[0][0])[k] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSortRounds; r++) {
+            if (32 * r >= per) break;
+            const int d = (key[r] >> (8 * pass)) & (kDigits - 1);
+            const bool have = first + 32 * r < n;
+            const unsigned same = __match_any_sync(full, have ? d : kDigits);
+            const int before = have ? s_cnt[warp][d] : 0;
+            __syncwarp();
+            at[r] = (unsigned short)(before + __popc(same & ((1u << lane) - 1u)));
+            if (have && lane == __ffs(same) - 1) s_cnt[warp][d] = (unsigned short)(before + __popc(same));
+            __syncwarp();
+        }
+        __syncthreads();
+        if (threadIdx.x < kDigits) {
+            int run = 0;
+            for (int w = 0; w < kSortWarps; w += 16) {
+                int c[16];
+#pragma unroll
+                for (int k = 0; k < 16; k++) c[k] = s_cnt[w + k][threadIdx.x];
+#pragma unroll
+                for (int k = 0; k < 16; k++) {
+                    s_cnt[w + k][threadIdx.x] = (unsigned short)run;
+                    run += c[k];
+                }
+            }
+            s_total[threadIdx.x] = run;
+        }
+        cluster.sync();
+        int all = 0, before = 0, incl = 0;
+        if (threadIdx.x < kDigits) {
+#pragma unroll
+            for (int b = 0; b < kSortBlocks; b++) {
+                const int c = *cluster.map_shared_rank(&s_total[threadIdx.x], b);
+                if (b < rank) before += c;
+                all += c;
+            }
+            incl = all;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(full, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (lane == 31) s_sum[warp] = incl;
+        }
+        __syncthreads();
+        if (threadIdx.x < kDigits) {
+            for (int w = 0; w < warp; w++) before += s_sum[w];
+            s_base[threadIdx.x] = before + incl - all;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSortRounds; r++) {
+            if (32 * r >= per || first + 32 * r >= n) break;
+            const int d = (key[r] >> (8 * pass)) & (kDigits - 1);
+            const int to = s_base[d] + s_cnt[warp][d] + at[r];
+            if (pass < 2) __stcg(&g->key[dst][to], key[r]);
+            __stcg(&g->order[dst][to], idx[r]);
+        }
+        __threadfence();
+        cluster.sync();  // the places are written, and every block's totals read
+    }
 }
 
 __global__ void __launch_bounds__(128) k_noalloc_runs(int n, const double *__restrict__ pos,
@@ -205,14 +315,14 @@ __device__ __forceinline__ void add_pair(const PassParams &p, const SumsInput &i
 // beyond |h| by more than the margin; NaNs are never rejected.
 //
 // What bounds it: the latency of a block's chain (run list, screen, evaluation),
-// not throughput. Measured on a clustered MFV set (whole call, the five launches
-// of the sort included): 57, 250 and 459 us at 1,000, 20,000 and 65,536 particles,
-// against 467, 5,731 and 18,294 us with one thread per target testing every pair
-// in FP64 (157 blocks of 128 at 20,000: four warps per multiprocessor, each
-// taking the sums for one or two of its lanes at a time). Four warps a block: 82,
-// 332, 544 us; eight at three blocks per multiprocessor (80 registers, spills):
-// 66, 292, 514 us. All pairs screened, without the order and the boxes: 27, 404
-// and 2,803 us.
+// not throughput. Measured on a clustered MFV set (whole call, sort included): 66,
+// 248 and 533 us at 1,000, 20,000 and 65,536 particles, against 473, 5,945 and
+// 18,300 us with one thread per target testing every pair in FP64 (157 blocks of
+// 128 at 20,000: four warps per multiprocessor, each taking the sums for one or two
+// of its lanes at a time). The alternatives were compared on another such set, at
+// 57, 250 and 459 us for this form: four warps a block 82, 332 and 544 us; eight at
+// three blocks per multiprocessor (80 registers, spills) 66, 292 and 514; all pairs
+// screened, without the order and the boxes, 27, 404 and 2,803.
 __global__ void __launch_bounds__(32 * kSlices, 2) k_noalloc_density_sums(PassParams p, int n,
                                                                           const double *__restrict__ pos,
                                                                           const double *__restrict__ vel,
@@ -419,18 +529,9 @@ extern "C" int gz_density_sums_noalloc(const gz_params *params, int n, const dou
     p.min_kernel_radius = params->min_kernel_radius;
     p.max_kernel_radius = params->max_kernel_radius;
     cudaStream_t s = (cudaStream_t)stream;
-    const unsigned blocks = (unsigned)((n + 127) / 128);
-    k_noalloc_keys<<<blocks, 128, 0, s>>>(n, pos, p.box, g->key[0], g->order[0]);
-    size_t need = 0;
-    if (cub::DeviceRadixSort::SortPairs(nullptr, need, g->key[0], g->key[1], g->order[0], g->order[1], n, 0, kKeyBits,
-                                        s) != cudaSuccess)
-        return GZ_ERR_CUDA;
-    if (need > kSortBytes) return GZ_ERR_INTERNAL;  // (0.4 MiB for the largest set)
-    if (cub::DeviceRadixSort::SortPairs(g->sort, need, g->key[0], g->key[1], g->order[0], g->order[1], n, 0, kKeyBits,
-                                        s) != cudaSuccess)
-        return GZ_ERR_CUDA;
-    k_noalloc_runs<<<blocks, 128, 0, s>>>(n, pos, h, g->order[1], g->pos, g->box);
-    const SumsWork w{g->order[1], g->pos, g->box};
+    k_noalloc_sort<<<kSortBlocks, 32 * kSortWarps, 0, s>>>(n, pos, p.box, g);
+    k_noalloc_runs<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(n, pos, h, g->order[0], g->pos, g->box);
+    const SumsWork w{g->order[0], g->pos, g->box};
     k_noalloc_density_sums<<<(unsigned)((n + kRun - 1) / kRun), 32 * kSlices, 0, s>>>(p, n, pos, vel, mass, h, w, acc,
                                                                                      pv);
     return cudaGetLastError() == cudaSuccess ? GZ_OK : GZ_ERR_CUDA;

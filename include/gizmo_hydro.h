@@ -354,7 +354,7 @@ int gz_density_sums(gz_context *ctx, const int *active, int n_active, double *ac
  *     the caller owns; rows follow the caller's order, every particle is a
  *     target and a candidate;
  *   - the only scratch is static device memory for GZ_NOALLOC_MAX_PARTICLES
- *     particles (3.1 MiB), held by every GPU that loads the library until the
+ *     particles (2.1 MiB), held by every GPU that loads the library until the
  *     process exits; n above that limit returns GZ_ERR_CAPACITY;
  *   - work is queued on `stream` (a cudaStream_t, NULL for the default
  *     stream) and the call returns without waiting: synchronise the stream
@@ -366,7 +366,9 @@ int gz_density_sums(gz_context *ctx, const int *active, int n_active, double *ac
  *     loaded on the device and the static memory is reserved, so it must come
  *     before the caller's memory pool reserves the device; setting
  *     CUDA_MODULE_LOADING=EAGER reserves it when the process first creates
- *     its CUDA context instead. A failed set-up returns GZ_ERR_CUDA;
+ *     its CUDA context instead. A failed set-up returns GZ_ERR_CUDA. Every call
+ *     launches the same kernels, whatever its n, so a first call on any set
+ *     loads all the code that later ones need;
  *   - every call on a device uses the same memory and rewrites it; two calls
  *     whose work overlaps on the GPU (different streams, no ordering between
  *     them) race on it and their results are undefined.
