@@ -61,6 +61,10 @@ static __device__ __align__(256) Scratch g_scratch;
 std::mutex g_setup_mutex;
 Scratch *g_scratch_ptr[kMaxDevices] = {};  // device address of g_scratch, per device
 
+// A particle index read from the scratch. It lies in [0, n) unless another call overlaps this one and rewrites the
+// scratch: the results are undefined then, but no access leaves the caller's arrays.
+__device__ __forceinline__ int own_index(int i, int n) { return (int)min((unsigned)i, (unsigned)(n - 1)); }
+
 // What the sums read of the scratch.
 struct SumsWork {
     const int *order;
@@ -206,7 +210,7 @@ __global__ void __launch_bounds__(128) k_noalloc_runs(int n, const double *__res
     float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf}, mag = 0.0f, h = 0.0f;
     bool nan = false;
     if (s < n) {
-        const size_t o = (size_t)order[s];
+        const size_t o = (size_t)own_index(order[s], n);
         const double hv = fabs(hs[o]);
         float f[3];
         for (int c = 0; c < 3; c++) {
@@ -348,7 +352,7 @@ __global__ void __launch_bounds__(32 * kSlices, 2) k_noalloc_density_sums(PassPa
     const int s = blockIdx.x * kRun + lane;
     const bool valid = s < n;
     const int sv = valid ? s : n - 1;  // a lane past the end follows the last target and stores nothing
-    const size_t i = (size_t)w.order[sv];
+    const size_t i = (size_t)own_index(w.order[sv], n);
     Target me;
     me.x = pos[3 * i]; me.y = pos[3 * i + 1]; me.z = pos[3 * i + 2];
     me.vx = vel[3 * i]; me.vy = vel[3 * i + 1]; me.vz = vel[3 * i + 2];
@@ -456,7 +460,7 @@ __global__ void __launch_bounds__(32 * kSlices, 2) k_noalloc_density_sums(PassPa
         while (__any_sync(full, pass != 0u)) {
             if (pass) {
                 const int k = __ffs(pass) - 1;
-                sh.scan.hit[hits++][threadIdx.x] = (unsigned short)__float_as_int(sh.scan.tile[slice][k].w);
+                sh.scan.hit[hits++][threadIdx.x] = (unsigned short)own_index(__float_as_int(sh.scan.tile[slice][k].w), n);
                 pass &= pass - 1u;
             }
             __syncwarp();

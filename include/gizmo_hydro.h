@@ -371,7 +371,8 @@ int gz_density_sums(gz_context *ctx, const int *active, int n_active, double *ac
  *     loads all the code that later ones need;
  *   - every call on a device uses the same memory and rewrites it; two calls
  *     whose work overlaps on the GPU (different streams, no ordering between
- *     them) race on it and their results are undefined.
+ *     them) race on it and their results are undefined (what they write stays
+ *     inside acc and pv).
  * The neighbour search takes every run of 32 particles against every other,
  * which is what bounds n. */
 #define GZ_NOALLOC_MAX_PARTICLES 65536

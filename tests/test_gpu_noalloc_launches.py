@@ -64,3 +64,31 @@ def test_every_call_launches_the_same_kernels():
     assert len(kernels[1]) >= 3
     for n in kernels:
         assert kernels[n] == kernels[1], n
+
+
+def test_overlapping_calls_stay_inside_their_arrays():
+    """Calls that overlap on the GPU have undefined results, and nothing more: a small set's outputs lie between
+    guards while calls of a large one rewrite the scratch under it, and a call by itself is right afterwards."""
+    import torch
+
+    n, guard = 1000, 70000
+    params, large = _inputs(65536)
+    _, small = _inputs(n)
+    _call(params, small)
+    torch.cuda.synchronize()
+    want, want_pv = small["acc"].clone(), small["pv"].clone()
+    acc = torch.full((n + 2 * guard, 14), -7.0, dtype=torch.float64, device="cuda")
+    pv = torch.full((n + 2 * guard, 3), -7.0, dtype=torch.float64, device="cuda")
+    inside = dict(small, acc=acc[guard:guard + n], pv=pv[guard:guard + n])
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(200):
+        for s, f in zip(streams, (large, inside)):
+            with torch.cuda.stream(s):
+                _call(params, f)
+    torch.cuda.synchronize()
+    for t in (acc, pv):
+        assert (t[:guard] == -7.0).all() and (t[guard + n:] == -7.0).all()
+    _call(params, inside)
+    torch.cuda.synchronize()
+    assert torch.equal(inside["acc"], want) and torch.equal(inside["pv"], want_pv)
