@@ -43,6 +43,9 @@ static_assert(kMaxParticles <= 65536, "a hit is a 16-bit particle index");
 
 // Bounding box of a run, rounded outward to FP32: lo.w the largest coordinate
 // magnitude, hi.w the largest |h|. A run that holds a NaN is given the whole space.
+// All lengths of the screen are in units of the box, so that their squares stay in
+// FP32's range whatever the unit of length is (unscaled, the squares of a box below
+// ~1e-19 are denormal, and the screen's slack no longer covers their rounding).
 struct RunBox {
     float4 lo, hi;
 };
@@ -52,7 +55,7 @@ struct RunBox {
 struct Scratch {
     unsigned key[2][kMaxParticles];
     int order[2][kMaxParticles];              // sorted -> caller's index: [0] after the sort
-    float4 pos[kMaxParticles];                // sorted FP32 positions; w: the caller's index
+    float4 pos[kMaxParticles];                // sorted FP32 positions in units of the box; w: the caller's index
     RunBox box[kMaxParticles / kRun];
 };
 static_assert(sizeof(Scratch) <= 2162688, "the documented size (2.1 MiB) is out of date");
@@ -202,8 +205,8 @@ __global__ void __cluster_dims__(kSortBlocks, 1, 1) __launch_bounds__(32 * kSort
 }
 
 __global__ void __launch_bounds__(128) k_noalloc_runs(int n, const double *__restrict__ pos,
-                                                      const double *__restrict__ hs, const int *__restrict__ order,
-                                                      float4 *out, RunBox *box)
+                                                      const double *__restrict__ hs, double unit,
+                                                      const int *__restrict__ order, float4 *out, RunBox *box)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const float inf = __int_as_float(0x7f800000);
@@ -211,10 +214,10 @@ __global__ void __launch_bounds__(128) k_noalloc_runs(int n, const double *__res
     bool nan = false;
     if (s < n) {
         const size_t o = (size_t)own_index(order[s], n);
-        const double hv = fabs(hs[o]);
+        const double hv = fabs(hs[o]) / unit;
         float f[3];
         for (int c = 0; c < 3; c++) {
-            const double v = pos[3 * o + c];
+            const double v = pos[3 * o + c] / unit;
             f[c] = __double2float_rn(v);
             lo[c] = __double2float_rd(v);
             hi[c] = __double2float_ru(v);
@@ -241,17 +244,17 @@ __global__ void __launch_bounds__(128) k_noalloc_runs(int n, const double *__res
 }
 
 // The most by which an FP32 separation can differ from the FP64 one, for
-// coordinates of magnitude up to m: each axis rounds two coordinates (2^-24 m
-// each), their difference (2^-24 2m) and the wrap (2^-24 (2m + box)), in all less
-// than 2^-24 (8m + 2 box) an axis and, over three axes and the rounding of the
-// squares, less than 2^-24 (16m + 8 box).
-__device__ __forceinline__ float screen_margin(float m, float box) { return 5.9604645e-8f * (16.0f * m + 8.0f * box); }
+// coordinates of magnitude up to m (units of the box): each axis divides two
+// coordinates by the box (2^-53 m each), rounds them (2^-24 m each), their difference
+// (2^-24 2m) and the wrap (2^-24 (2m + 1)), in all less than 2^-24 (8m + 2) an axis
+// and, over three axes and the rounding of the squares, less than 2^-24 (16m + 8).
+__device__ __forceinline__ float screen_margin(float m) { return 5.9604645e-8f * (16.0f * m + 8.0f); }
 
-// distance of the interval [a, b] of coordinate differences to the nearest of 0 and +-box, where a pair's
-// minimum image on one axis is measured from
-__device__ __forceinline__ float axis_distance(float a, float b, float box)
+// distance of the interval [a, b] of coordinate differences to the nearest of 0 and +-1 (the box), where a
+// pair's minimum image on one axis is measured from
+__device__ __forceinline__ float axis_distance(float a, float b)
 {
-    const float d0 = fmaxf(a, -b), dp = fmaxf(a - box, box - b), dm = fmaxf(a + box, -box - b);
+    const float d0 = fmaxf(a, -b), dp = fmaxf(a - 1.0f, 1.0f - b), dm = fmaxf(a + 1.0f, -1.0f - b);
     return fmaxf(fminf(d0, fminf(dp, dm)), 0.0f);
 }
 
@@ -400,7 +403,7 @@ __global__ void __launch_bounds__(32 * kSlices, 2) k_noalloc_density_sums(PassPa
 
     const float4 mf = w.pos[sv];
     const RunBox mine = w.box[blockIdx.x];
-    const float boxf = (float)p.box, hf = __double2float_ru(fabs(hd));
+    const float hf = __double2float_ru(fabs(hd) / p.box);
     const int runs = (n + kRun - 1) / kRun;
     // the runs the targets can reach
     if (threadIdx.x == 0) s_top = 0u;
@@ -412,10 +415,10 @@ __global__ void __launch_bounds__(32 * kSlices, 2) k_noalloc_density_sums(PassPa
         if (q < runs) {
             const RunBox b = w.box[q];
             top = b.lo.w;
-            const float R = mine.hi.w + screen_margin(fmaxf(mine.lo.w, top), boxf);
-            const float gx = axis_distance(mine.lo.x - b.hi.x, mine.hi.x - b.lo.x, boxf);
-            const float gy = axis_distance(mine.lo.y - b.hi.y, mine.hi.y - b.lo.y, boxf);
-            const float gz = axis_distance(mine.lo.z - b.hi.z, mine.hi.z - b.lo.z, boxf);
+            const float R = mine.hi.w + screen_margin(fmaxf(mine.lo.w, top));
+            const float gx = axis_distance(mine.lo.x - b.hi.x, mine.hi.x - b.lo.x);
+            const float gy = axis_distance(mine.lo.y - b.hi.y, mine.hi.y - b.lo.y);
+            const float gz = axis_distance(mine.lo.z - b.hi.z, mine.hi.z - b.lo.z);
             in = !(gx * gx + gy * gy + gz * gz > R * R * 1.000001f);
         }
         const unsigned bal = __ballot_sync(full, in);
@@ -435,7 +438,7 @@ __global__ void __launch_bounds__(32 * kSlices, 2) k_noalloc_density_sums(PassPa
         if (in) s_run[at + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)q;
     }
     __syncthreads();
-    const float hi = hf + screen_margin(fmaxf(__uint_as_float(s_top), mine.lo.w), boxf);
+    const float hi = hf + screen_margin(fmaxf(__uint_as_float(s_top), mine.lo.w));
     const float hi2 = hi * hi * 1.000001f;
     for (int q0 = 0; q0 < reached; q0 += kSlices) {
         const int ql = q0 + lane / kShare;
@@ -448,11 +451,11 @@ __global__ void __launch_bounds__(32 * kSlices, 2) k_noalloc_density_sums(PassPa
 #pragma unroll
         for (int k = 0; k < 32; k++) {
             const float4 q = sh.scan.tile[slice][k];
-            // the minimum image's magnitude: |d|, or box - |d| beyond half the box (squared below)
+            // the minimum image's magnitude: |d|, or 1 - |d| beyond half the box (squared below)
             float dx = fabsf(mf.x - q.x), dy = fabsf(mf.y - q.y), dz = fabsf(mf.z - q.z);
-            dx = fminf(dx, boxf - dx);
-            dy = fminf(dy, boxf - dy);
-            dz = fminf(dz, boxf - dz);
+            dx = fminf(dx, 1.0f - dx);
+            dy = fminf(dy, 1.0f - dy);
+            dz = fminf(dz, 1.0f - dz);
             const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
             if (!(r2 > hi2)) pass |= 1u << k;
         }
@@ -534,7 +537,7 @@ extern "C" int gz_density_sums_noalloc(const gz_params *params, int n, const dou
     p.max_kernel_radius = params->max_kernel_radius;
     cudaStream_t s = (cudaStream_t)stream;
     k_noalloc_sort<<<kSortBlocks, 32 * kSortWarps, 0, s>>>(n, pos, p.box, g);
-    k_noalloc_runs<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(n, pos, h, g->order[0], g->pos, g->box);
+    k_noalloc_runs<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(n, pos, h, p.box, g->order[0], g->pos, g->box);
     const SumsWork w{g->order[0], g->pos, g->box};
     k_noalloc_density_sums<<<(unsigned)((n + kRun - 1) / kRun), 32 * kSlices, 0, s>>>(p, n, pos, vel, mass, h, w, acc,
                                                                                      pv);

@@ -80,3 +80,21 @@ def test_a_nan_position_reaches_every_sum():
     wl.pos[500, 1] = np.nan
     acc, _ = _noalloc(wl)
     assert np.isnan(acc[:, 0]).all()
+
+
+@pytest.mark.parametrize("shift", [-200, -70, 70, 200])
+def test_the_unit_of_length_does_not_matter(shift):
+    """Lengths scaled by a power of two scale every sum by one: no rounding differs, so neither does any decision of
+    the screen. (At 2^-70 the squares of FP32 separations would be denormal, at 2^70 infinite.)"""
+    import copy
+
+    want = _subset(3000)
+    wl = copy.deepcopy(want)
+    f = 2.0 ** shift
+    wl.pos, wl.h, wl.params.box_size = wl.pos * f, wl.h * f, want.params.box_size * f
+    a, apv = _noalloc(want)
+    b, bpv = _noalloc(wl)
+    # W, m W ~ 1 / h^3; 3 W / h + u dW/du and dW/dr dx dv / r ~ 1 / h^4; x x W ~ 1 / h; x W ~ 1 / h^2
+    for c, power in enumerate([3, 3, 4, 4] + [1] * 6 + [2] * 3):
+        assert np.array_equal(b[:, c] * f ** power, a[:, c]), c
+    assert np.array_equal(bpv * f ** 3, apv)
