@@ -202,8 +202,11 @@ __global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads
             split_node(keys, node, parent, tb, beg + i, L, total, cap, leaf_max, split_levels, box_of, root_of, lane, mask);
         __threadfence();
         cl.sync();
+        // The level's own count is final here; whether it passed the capacity is told from it and not from
+        // tb->fail, which a block already in the next level may set: every thread leaves at the same level.
+        const int made = *(volatile int *)&tb->next[L];
         beg = total;
-        cnt = *(volatile int *)&tb->fail ? 0 : *(volatile int *)&tb->next[L];
+        cnt = (long long)total + made > cap ? 0 : made;
         total += cnt;
         L++;
     }

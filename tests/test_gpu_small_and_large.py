@@ -36,6 +36,27 @@ def test_rows_of_deep_trees(n):
     assert np.array_equal(off, ooff) and np.array_equal(nbr, onbr)
 
 
+@pytest.mark.parametrize("n, nested", [(20000, False), (65536, False), (65536, True), (90000, False), (300000, True)])
+def test_rows_of_trees_that_outgrow_their_nodes(n, nested):
+    """Leaves of at most 8 particles make more nodes than are held for the set (a quarter of its particles): the
+    device build stops in mid-level, in the cluster or in a level's launch, and the tree is built level by level."""
+    rng = np.random.default_rng(n)
+    wl = ics.sedov(4)
+    pos = _nested(n, rng) if nested else rng.random((n, 3))
+    z, one = np.zeros((n, 3)), np.ones(n)
+    h = np.full(n, 1e-7 if nested else 0.6 * n ** (-1 / 3))
+    act = rng.choice(n, size=500, replace=False).astype(np.int32)
+    with HydroPass(wl.params) as hp:
+        hp.set_tuning(8, 2.5)
+        for _ in range(3):
+            hp.upload(pos, z, one / n, one, one * 2.0 ** -8, h)
+            off, nbr = hp.neighbors(0, act)
+            for r, i in enumerate(act):
+                d = pos - pos[i]
+                d -= np.round(d)
+                assert np.array_equal(nbr[off[r]:off[r + 1]], np.nonzero((d ** 2).sum(1) < h[i] ** 2)[0])
+
+
 def test_box_sets_with_empty_boxes():
     a, b = ics.shock_tube(8, seed=5), ics.sedov(9, seed=6)
     counts = [0, a.n, 0, 0, b.n, 0]
