@@ -328,6 +328,7 @@ __global__ void __launch_bounds__(128) k_tree_up(int n_nodes, const int *__restr
                 if (!last) p = -1;
             }
         }
+        __syncwarp(mask);  // what lane 0 has seen of the siblings' boxes (the counter, its fences), its lanes see too
         p = __shfl_sync(mask, p, 0, kNodeLanes);
         if (p < 0) return;
         i = p;
