@@ -2478,6 +2478,21 @@ static bool pinned_buffer(gz_context *c, size_t bytes)
     return true;
 }
 
+// May the host write fields f[first, last) itself? Not to device memory, which the
+// runtime's copy has its own answer to.
+static bool host_writable(const std::vector<OutField> &f, size_t first, size_t last)
+{
+    for (size_t i = first; i < last; i++) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, f[i].dst) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (a.type == cudaMemoryTypeDevice) return false;
+    }
+    return true;
+}
+
 // gz_download into host arrays through the staging buffer, or (to_device)
 // straight into the caller's device arrays (gz_download_device). The host
 // form scatters as many fields as the staging holds (up to 16 doubles per
@@ -2517,7 +2532,7 @@ static int download_to(gz_context *c, const gz_outputs *o, bool to_device)
         }
         scatter_fields(c, f, first, last, s, at);
         GZ_CUDA(c, cudaGetLastError());
-        if (used <= kPinnedBytes && pinned_buffer(c, used)) {
+        if (used <= kPinnedBytes && pinned_buffer(c, used) && host_writable(f, first, last)) {
             GZ_CUDA(c, cudaMemcpyAsync(c->pinned, c->dl.p, used, cudaMemcpyDeviceToHost, s));
             GZ_CUDA(c, cudaStreamSynchronize(s));
             for (size_t i = first; i < last; i++)

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from gizmo_b200 import ics
-from gizmo_b200.hydro import HydroPass
+from gizmo_b200.hydro import GizmoHydroError, HydroPass
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -127,3 +127,30 @@ def test_repeated_downloads_are_equal():
                 got = hp.download()
                 for k in want:
                     assert np.array_equal(got[k], want[k]), k
+
+
+def test_a_host_download_to_device_memory_has_the_runtimes_answer_at_any_time():
+    """gz_download is for host arrays. What the runtime's copy answers to a device address (an error, or the copy)
+    is what a context answers, new or in use: it never writes there from the host."""
+    import torch
+
+    wl = ics.shock_tube(8, seed=2)
+    dst = torch.zeros(wl.n, dtype=torch.float64, device="cuda")
+    answers = []
+    with HydroPass(wl.params) as hp:
+        hp.upload_workload(wl)
+        hp.full_pass()
+        rho = hp.download(["rho"])["rho"]
+        for k in range(12):
+            if k in (0, 11):
+                dst.zero_()
+                torch.cuda.synchronize()
+                try:
+                    hp.download_raw({"rho": dst.data_ptr()})
+                    answers.append(np.array_equal(dst.cpu().numpy(), rho))
+                except GizmoHydroError as e:
+                    answers.append(e.code)
+            hp.upload_workload(wl)
+            hp.full_pass()
+            hp.download()
+    assert answers[0] == answers[1] and answers[0] is not False, answers
