@@ -224,11 +224,13 @@ int fail(gz_context *c, int code, const char *what)
 
 template <typename T> T *ptr(DevBuf &b) { return (T *)b.p; }
 
-// The buffer at `bytes` or more; false when it cannot be had (the error is cleared).
+// The buffer at `bytes` or more; false, and cudaMalloc's answer in `why`, when it cannot be
+// had. (A lack of memory is cleared from the runtime; any other answer, an earlier fault
+// among them, is left there.)
 // A buffer that has to grow grows by a quarter more than asked: the row totals of an
 // evolving set creep up from step to step, and freeing and allocating the row and
 // flux buffers in each of them cost 2 to 9 ms of a 2 ms step of 64,000 cells.
-bool try_ensure(DevBuf &b, size_t bytes)
+bool try_ensure(DevBuf &b, size_t bytes, cudaError_t *why = nullptr)
 {
     if (b.bytes >= bytes && b.p) return true;
     const size_t exact = bytes > 0 ? bytes : 16;
@@ -236,15 +238,17 @@ bool try_ensure(DevBuf &b, size_t bytes)
     if (b.p) cudaFree(b.p);
     b.p = nullptr;
     b.bytes = 0;
-    if (cudaMalloc(&b.p, want) != cudaSuccess) {
-        cudaGetLastError();  // clear the allocation failure
-        b.p = nullptr;
+    cudaError_t e = cudaMalloc(&b.p, want);
+    if (e == cudaErrorMemoryAllocation && want > exact) {
+        cudaGetLastError();
         want = exact;
-        if (cudaMalloc(&b.p, want) != cudaSuccess) {
-            cudaGetLastError();
-            b.p = nullptr;
-            return false;
-        }
+        e = cudaMalloc(&b.p, want);
+    }
+    if (e != cudaSuccess) {
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+        if (why) *why = e;
+        b.p = nullptr;
+        return false;
     }
     b.bytes = want;
     return true;
@@ -253,8 +257,11 @@ bool try_ensure(DevBuf &b, size_t bytes)
 // like try_ensure(), and a failed allocation is an error of the context
 int ensure(gz_context *c, DevBuf &b, size_t bytes)
 {
-    if (!try_ensure(b, bytes)) return fail(c, GZ_ERR_CUDA, "out of device memory");
-    return 0;
+    cudaError_t why = cudaSuccess;
+    if (try_ensure(b, bytes, &why)) return 0;
+    char msg[200];
+    snprintf(msg, sizeof(msg), "cudaMalloc of %zu bytes: %s", bytes, cudaGetErrorString(why));
+    return fail(c, GZ_ERR_CUDA, msg);
 }
 
 void release(DevBuf &b)
