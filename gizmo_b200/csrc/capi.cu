@@ -6,6 +6,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -95,6 +96,7 @@ struct gz_context {
     DevBuf pad_over, pad_list, pad_sum, pad_counts;  // padded single-walk density rows
     DevBuf s_acnt, s_bcnt, s_tmp;    // symmetric rows derived from the density rows
     DevBuf pflux;                    // force pass evaluating each pair once: the flux per row entry
+    std::vector<DevBuf *> in_use;    // pair buffers that make_room must not give back (Using)
     // symmetric rows (shared by gradients and force)
     DevBuf s_off, s_nbr, s_counts;
     long long s_nbr_cap = 0;
@@ -224,22 +226,87 @@ int fail(gz_context *c, int code, const char *what)
 
 template <typename T> T *ptr(DevBuf &b) { return (T *)b.p; }
 
-// The buffer at `bytes` or more; false, and cudaMalloc's answer in `why`, when it cannot be
-// had. (A lack of memory is cleared from the runtime; any other answer, an earlier fault
-// among them, is left there.)
-// A buffer that has to grow grows by a quarter more than asked: the row totals of an
-// evolving set creep up from step to step, and freeing and allocating the row and
-// flux buffers in each of them cost 2 to 9 ms of a 2 ms step of 64,000 cells.
-bool try_ensure(DevBuf &b, size_t bytes, cudaError_t *why = nullptr)
+void release(DevBuf &b)
 {
-    if (b.bytes >= bytes && b.p) return true;
-    const size_t exact = bytes > 0 ? bytes : 16;
-    size_t want = b.p ? exact + exact / 4 : exact;
     if (b.p) cudaFree(b.p);
     b.p = nullptr;
     b.bytes = 0;
+}
+
+// The buffers whose size follows the pair counts and whose contents no call leaves to a later
+// one: the pair fluxes, the two queues and the scratch of the symmetric rows. (The symmetric
+// rows themselves are left to the force pass while sym_valid is set.)
+std::array<DevBuf *, 5> pair_buffers(gz_context *c) { return {&c->pflux, &c->rq, &c->dq, &c->s_tmp, &c->s_nbr}; }
+
+// Marks pair buffers as in use while the object lives: make_room leaves them alone.
+struct Using {
+    gz_context *c;
+    size_t before;
+    Using(gz_context *ctx, std::initializer_list<DevBuf *> b) : c(ctx), before(ctx->in_use.size())
+    {
+        c->in_use.insert(c->in_use.end(), b.begin(), b.end());
+    }
+    ~Using() { c->in_use.resize(before); }
+    Using(const Using &) = delete;
+};
+
+// Gives back the pair buffers that are not in use, and what the symmetric rows hold beyond
+// their entries, to make room for buffer `but`. Returns whether anything was given back.
+bool make_room(gz_context *c, const DevBuf *but)
+{
+    bool any = false;
+    for (DevBuf *b : pair_buffers(c)) {
+        if (!b->p || b == but || std::find(c->in_use.begin(), c->in_use.end(), b) != c->in_use.end()) continue;
+        const size_t keep = (b == &c->s_nbr && c->sym_valid) ? sizeof(int) * (size_t)c->pairs_symmetric : 0;
+        if (keep && b->bytes <= keep) continue;
+        DevBuf kept;
+        if (keep) {  // (last in the list: the others have made the room for the copy)
+            if (cudaMalloc(&kept.p, keep) != cudaSuccess) {
+                cudaGetLastError();
+                continue;
+            }
+            kept.bytes = keep;
+            if (cudaMemcpyAsync(kept.p, b->p, keep, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess ||
+                cudaStreamSynchronize(c->stream) != cudaSuccess) {
+                release(kept);
+                continue;
+            }
+        }
+        release(*b);
+        *b = kept;
+        any = true;
+    }
+    c->s_nbr_cap = std::min(c->s_nbr_cap, (long long)(c->s_nbr.bytes / sizeof(int)));
+    return any;
+}
+
+// The buffer at `bytes` or more; false, and cudaMalloc's answer in `why`, when it cannot be
+// had. (A lack of memory is cleared from the runtime; any other answer, an earlier fault
+// among them, is left there.)
+//
+// Buffers have the size that was asked for, but one that has to grow by less than a quarter
+// takes a quarter more than asked if it is a pair buffer or small: the row totals of an
+// evolving set creep up from step to step, and freeing and allocating these buffers in each
+// of them made a step of 64,000 cells that takes 1.6 ms take 3.5. That room costs nothing when
+// memory is short: small buffers hold 100 MB of it at most, in all, and pair buffers are given
+// back (and come back at their exact sizes) before an allocation fails.
+constexpr size_t kSmallBuffer = 4 << 20;
+bool try_ensure(gz_context *c, DevBuf &b, size_t bytes, cudaError_t *why = nullptr)
+{
+    if (b.bytes >= bytes && b.p) return true;
+    const size_t exact = bytes > 0 ? bytes : 16;
+    const auto pair = pair_buffers(c);
+    const bool creeps = b.p && exact <= b.bytes + b.bytes / 4 &&
+                        (exact <= kSmallBuffer || std::find(pair.begin(), pair.end(), &b) != pair.end());
+    size_t want = creeps ? exact + exact / 4 : exact;
+    release(b);
     cudaError_t e = cudaMalloc(&b.p, want);
     if (e == cudaErrorMemoryAllocation && want > exact) {
+        cudaGetLastError();
+        want = exact;
+        e = cudaMalloc(&b.p, want);
+    }
+    if (e == cudaErrorMemoryAllocation && make_room(c, &b)) {
         cudaGetLastError();
         want = exact;
         e = cudaMalloc(&b.p, want);
@@ -258,17 +325,28 @@ bool try_ensure(DevBuf &b, size_t bytes, cudaError_t *why = nullptr)
 int ensure(gz_context *c, DevBuf &b, size_t bytes)
 {
     cudaError_t why = cudaSuccess;
-    if (try_ensure(b, bytes, &why)) return 0;
+    if (try_ensure(c, b, bytes, &why)) return 0;
     char msg[200];
     snprintf(msg, sizeof(msg), "cudaMalloc of %zu bytes: %s", bytes, cudaGetErrorString(why));
     return fail(c, GZ_ERR_CUDA, msg);
 }
 
-void release(DevBuf &b)
+// Several buffers that are needed together, none of whose contents is: when one cannot be
+// had, all are given back and taken again at their exact sizes. False when that fails too.
+struct Need {
+    DevBuf *b;
+    size_t bytes;
+};
+bool ensure_together(gz_context *c, const std::vector<Need> &need)
 {
-    if (b.p) cudaFree(b.p);
-    b.p = nullptr;
-    b.bytes = 0;
+    Using use(c, {});
+    for (const Need &x : need) c->in_use.push_back(x.b);
+    for (int attempt = 0;; attempt++) {
+        bool ok = true;
+        for (const Need &x : need) ok = ok && try_ensure(c, *x.b, x.bytes);
+        if (ok || attempt) return ok;
+        for (const Need &x : need) release(*x.b);
+    }
 }
 
 PassParams make_pass_params(const gz_params &p)
@@ -990,11 +1068,10 @@ int sym_rows_from_density(gz_context *c)
     long long total = 0;
     if (exclusive_scan_counts(c, n, c->s_counts, c->s_off, &total)) return c->err;
     if (total > (long long)INT32_MAX * 4) return fail(c, GZ_ERR_CAPACITY, "neighbour rows exceed capacity");
-    if (ensure(c, c->s_tmp, sizeof(int) * (size_t)std::max(total, 1ll))) return c->err;
-    if (total > c->s_nbr_cap || !c->s_nbr.p) {
-        if (ensure(c, c->s_nbr, sizeof(int) * (size_t)std::max(total, 1ll))) return c->err;
-        c->s_nbr_cap = (long long)(c->s_nbr.bytes / sizeof(int));
-    }
+    const size_t bytes = sizeof(int) * (size_t)std::max(total, 1ll);
+    const bool room = ensure_together(c, {{&c->s_tmp, bytes}, {&c->s_nbr, bytes}});
+    c->s_nbr_cap = (long long)(c->s_nbr.bytes / sizeof(int));
+    if (!room) return fail(c, GZ_ERR_CUDA, "out of memory for the symmetric rows");
     GZ_CUDA(c, cudaMemsetAsync(c->s_bcnt.p, 0, sizeof(int) * N, s));  // reused as the B cursors
     sym_scatter(n, ptr<long long>(c->d_beg), ptr<int>(c->d_nbr), ptr<int>(c->s_acnt), ptr<long long>(c->s_off),
                 ptr<int>(c->s_bcnt), ptr<int>(c->s_tmp), s);
@@ -1010,15 +1087,16 @@ int sym_rows_from_density(gz_context *c)
 // stage of 1% of 2M particles, 4.62 against 2.70 for 10% of 1M): cap slots per target in scratch
 // (the walk counts every row in full), their counts scanned into offsets, the
 // rows copied to their places, and the few longer than cap filled by a walk of
-// their own. `fits` is false when there is no room for the slots: nothing is
-// built then.
+// their own. `fits` is false when there is no room for the slots beside the rows:
+// nothing is built then.
 int sym_rows_one_walk(gz_context *c, int rows, long long *total, bool *fits)
 {
     cudaStream_t s = c->stream;
     const int cap = 32 * (int)std::ceil(c->row_slots * c->prm.des_num_ngb / 32.0);
     const long long slots = (long long)rows * cap;
-    *fits = slots <= (long long)INT32_MAX && try_ensure(c->s_tmp, sizeof(int) * (size_t)slots);
+    *fits = slots <= (long long)INT32_MAX && try_ensure(c, c->s_tmp, sizeof(int) * (size_t)slots);
     if (!*fits) return 0;
+    Using use(c, {&c->s_tmp});
     const size_t R = (size_t)rows;
     if (ensure(c, c->s_counts, sizeof(long long) * R) || ensure(c, c->s_off, sizeof(long long) * (R + 1)) ||
         ensure(c, c->work, sizeof(int)) || ensure(c, c->pad_list, sizeof(int) * R) ||
@@ -1043,7 +1121,12 @@ int sym_rows_one_walk(gz_context *c, int rows, long long *total, bool *fits)
     GZ_CUDA(c, cudaStreamSynchronize(s));
     c->launches += 2;
     if (*total > (long long)INT32_MAX * 4) return fail(c, GZ_ERR_CAPACITY, "neighbour rows exceed capacity");
-    if (grow_keep(c, c->s_nbr, c->s_nbr_cap, 0, *total)) return c->err;
+    *fits = try_ensure(c, c->s_nbr, sizeof(int) * (size_t)*total);
+    c->s_nbr_cap = (long long)(c->s_nbr.bytes / sizeof(int));
+    if (!*fits) {  // the slots stand in the way of the rows
+        release(c->s_tmp);
+        return 0;
+    }
     copy_rows(rows, counts, off, cap, ptr<int>(c->s_tmp), ptr<int>(c->s_nbr), s);
     c->launches++;
     if (n_long > 0) {
@@ -1058,6 +1141,7 @@ int sym_rows_one_walk(gz_context *c, int rows, long long *total, bool *fits)
 
 int build_sym_rows(gz_context *c, int rows, bool all)
 {
+    c->sym_valid = false;  // until the new rows are complete
     if (all && c->dens_all && rows == c->n && c->n > 0) {
         if (sym_rows_from_density(c)) return c->err;
     } else {
@@ -1460,23 +1544,9 @@ int graph_buffers(gz_context *c, long long *sym_cap, long long *rq_cap, bool wit
         ensure(c, c->g_over_off, sizeof(long long) * N) || ensure(c, c->s_acnt, sizeof(int) * N) ||
         ensure(c, c->s_bcnt, sizeof(int) * N) || ensure(c, c->s_counts, sizeof(long long) * N) ||
         ensure(c, c->s_off, sizeof(long long) * (N + 1)) || ensure(c, c->refined, sizeof(unsigned long long)) ||
-        ensure(c, c->deferred, sizeof(unsigned long long)) ||
-        ensure(c, c->dq, sizeof(RefineItem) * (size_t)deferred_cap(sc)) || ensure(c, c->keep, N) || ensure(c, c->regrow, N) ||
+        ensure(c, c->deferred, sizeof(unsigned long long)) || ensure(c, c->keep, N) || ensure(c, c->regrow, N) ||
         ensure(c, c->g_sel, sizeof(int) * 2 * (N / kSelChunk + 1)))
         return c->err;
-    // the large buffers: without room for them the pass runs plain (which
-    // allocates what it needs again)
-    if (c->d_nbr_cap < nbr_need || !c->d_nbr.p) {
-        if (!try_ensure(c->d_nbr, sizeof(int) * (size_t)nbr_need)) { c->d_nbr_cap = 0; return kNoRoom; }
-        c->d_nbr_cap = nbr_need;
-    }
-    if (!try_ensure(c->s_tmp, sizeof(int) * (size_t)sc)) return kNoRoom;
-    if ((long long)(c->s_nbr.bytes / sizeof(int)) < sc || !c->s_nbr.p) {
-        if (!try_ensure(c->s_nbr, sizeof(int) * (size_t)sc)) { c->s_nbr_cap = 0; return kNoRoom; }
-        c->s_nbr_cap = (long long)(c->s_nbr.bytes / sizeof(int));
-    }
-    if (!try_ensure(c->pflux, pair_flux_bytes(mixed) * (size_t)sc)) return kNoRoom;
-    if (mixed && !try_ensure(c->rq, sizeof(RefineItem) * (size_t)rq)) return kNoRoom;
     size_t tmp = 0, tmp_sort = 0;
     cub::DeviceScan::InclusiveSum(nullptr, tmp, ptr<long long>(c->s_counts), ptr<long long>(c->s_off) + 1, n,
                                   c->stream);
@@ -1491,6 +1561,20 @@ int graph_buffers(gz_context *c, long long *sym_cap, long long *rq_cap, bool wit
             return c->err;
     }
     if (ensure(c, c->cub_tmp, std::max(tmp, tmp_sort))) return c->err;
+    // the large buffers, last: without room for them the pass runs plain (which
+    // allocates what it needs again)
+    c->sym_valid = c->dens_all = false;  // (both kinds of rows are built again, either way)
+    std::vector<Need> large = {{&c->dq, sizeof(RefineItem) * (size_t)deferred_cap(sc)},
+                               {&c->d_nbr, sizeof(int) * (size_t)nbr_need},
+                               {&c->s_tmp, sizeof(int) * (size_t)sc},
+                               {&c->s_nbr, sizeof(int) * (size_t)sc},
+                               {&c->pflux, pair_flux_bytes(mixed) * (size_t)sc}};
+    if (mixed) large.push_back({&c->rq, sizeof(RefineItem) * (size_t)rq});
+    const bool room = ensure_together(c, large);
+    c->s_nbr_cap = (long long)(c->s_nbr.bytes / sizeof(int));
+    c->d_nbr_cap = std::min(c->d_nbr_cap, (long long)(c->d_nbr.bytes / sizeof(int)));
+    if (!room) return kNoRoom;
+    c->d_nbr_cap = std::max(c->d_nbr_cap, nbr_need);
     *sym_cap = std::min<long long>({sc, (long long)(c->s_nbr.bytes / sizeof(int)), (long long)(c->s_tmp.bytes / sizeof(int)),
                                     (long long)(c->pflux.bytes / pair_flux_bytes(mixed))});
     *rq_cap = rq;
@@ -2302,7 +2386,6 @@ int gz_hydro_force(gz_context *c, const int *active, int n_active)
         c->sym_all = (active == nullptr);
         c->sym_active.assign(active ? active : (const int *)nullptr, active ? active + n_active : (const int *)nullptr);
     }
-    Csr rows{ptr<long long>(c->s_off), ptr<int>(c->s_nbr)};
     Particles ps = view(c);
     if (c->have_bins && c->n > 0) GZ_CUDA(c, cudaMemsetAsync(c->wakeup.p, 0, sizeof(int) * (size_t)c->n, c->stream));
     force_preloop(c->pp, ps, ptr<int>(c->targets), na, c->stream);
@@ -2313,29 +2396,34 @@ int gz_hydro_force(gz_context *c, const int *active, int n_active)
     // again in FP64 there); the FP64 form otherwise evaluates the rows in place.
     const int mixed = c->prm.precision == GZ_PRECISION_MIXED;
     const bool all = active == nullptr && na == c->n && c->n > 0;
-    void *flux = nullptr;
-    if (na > 0 && try_ensure(c->pflux, pair_flux_bytes(mixed) * (size_t)std::max(c->pairs_symmetric, 1ll)))
-        flux = c->pflux.p;
-    if (mixed && na > 0 && !flux) return fail(c, GZ_ERR_CAPACITY, "mixed-form force pass: no room for the pair fluxes");
     // Mixed form: queue room for one pair in 8 of the pass (about one in 700 is
     // queued on the Plummer mixture, one in 130 on the log-normal field). A pass
     // over every particle that queued more runs again with room for all of
     // them; an active subset cannot (its j-side mass writes would count twice).
     long long cap = mixed ? std::max(65536ll, c->pairs_symmetric / 8) : 0;
+    if (ensure(c, c->refined, sizeof(unsigned long long)) || ensure(c, c->deferred, sizeof(unsigned long long)))
+        return c->err;
+    bool room = false;
+    for (long long items : {deferred_cap(c->pairs_symmetric), 1024ll}) {  // (fewer than are deferred: the rows are scanned)
+        std::vector<Need> need = {{&c->dq, sizeof(RefineItem) * (size_t)items},
+                                  {&c->pflux, pair_flux_bytes(mixed) * (size_t)std::max(c->pairs_symmetric, 1ll)}};
+        if (mixed) need.push_back({&c->rq, sizeof(RefineItem) * (size_t)cap});
+        if ((room = ensure_together(c, need))) break;
+    }
+    void *flux = room ? c->pflux.p : nullptr;
+    if (mixed && !room) return fail(c, GZ_ERR_CAPACITY, "mixed-form force pass: no room for the pair fluxes");
+    Using use(c, {&c->pflux, &c->dq, &c->s_nbr});
+    const Csr rows{ptr<long long>(c->s_off), ptr<int>(c->s_nbr)};
     unsigned long long refined = 0;
     for (int attempt = 0;; attempt++) {
         RefineQueue q{nullptr, nullptr, 0};
         if (mixed) {
-            if (ensure(c, c->refined, sizeof(unsigned long long)) || ensure(c, c->rq, sizeof(RefineItem) * (size_t)cap))
-                return c->err;
+            if (ensure(c, c->rq, sizeof(RefineItem) * (size_t)cap)) return c->err;
             GZ_CUDA(c, cudaMemsetAsync(c->refined.p, 0, sizeof(unsigned long long), c->stream));
             q = RefineQueue{ptr<RefineItem>(c->rq), ptr<unsigned long long>(c->refined), cap};
         }
         RefineQueue dq{nullptr, nullptr, 0};
         if (flux) {
-            if (ensure(c, c->deferred, sizeof(unsigned long long)) ||
-                ensure(c, c->dq, sizeof(RefineItem) * (size_t)deferred_cap(c->pairs_symmetric)))
-                return c->err;
             GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), c->stream));
             dq = RefineQueue{ptr<RefineItem>(c->dq), ptr<unsigned long long>(c->deferred),
                              (long long)(c->dq.bytes / sizeof(RefineItem))};
@@ -2580,7 +2668,7 @@ static int download_async(gz_context *c, const gz_outputs *o)
     if (c->out_pending) GZ_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_out_done, 0));
     if (!c->dstage.p || c->dstage.bytes < total) {
         if (c->out_pending) GZ_CUDA(c, cudaEventSynchronize(c->ev_out_done));
-        if (!try_ensure(c->dstage, total)) return download_to(c, o, false);  // no room: the plain download
+        if (!try_ensure(c, c->dstage, total)) return download_to(c, o, false);  // no room: the plain download
     }
     cudaStream_t s = c->stream;
     std::vector<void *> to;

@@ -5,7 +5,7 @@ import contextlib
 import numpy as np
 import pytest
 
-from gizmo_b200 import ics
+from gizmo_b200 import abi, ics
 from gizmo_b200.hydro import GizmoHydroError, HydroPass
 
 pytestmark = pytest.mark.gpu
@@ -57,3 +57,90 @@ def test_a_failed_allocation_reports_cudas_own_words_and_can_be_repeated():
         got = hp.download()
         for k in want:
             assert np.array_equal(got[k], want[k]), k
+
+
+def _crept(precision, n=600_000):
+    """A context whose pair buffers have grown by a little and hold room to grow further, with its last results."""
+    p = ics.sedov(4, precision=precision).params
+    hp = HydroPass(p)
+    hp.upload(**_uniform(n))
+    hp.full_pass()
+    p.des_num_ngb = 33.0
+    hp.set_params(p)
+    hp.restage()
+    hp.full_pass()
+    return hp, hp.status()
+
+
+@pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_MIXED], ids=["fp64", "mixed"])
+def test_room_to_grow_is_given_back_before_an_allocation_fails(precision):
+    n = 600_000
+    flux = {abi.PRECISION_FP64: 64, abi.PRECISION_MIXED: 32}[precision]
+    names = ["h", "rho", "accel", "dudt"]
+    hp, _ = _crept(precision, n)
+    with hp:
+        want = hp.download(names)
+    hp, st = _crept(precision, n)  # (a download takes staging: this one has made none)
+    with hp:
+        sized = hp.status()["device_bytes"]
+        room = flux * st["pairs_symmetric"] // 4  # what the fluxes hold beyond their entries, at least
+        assert room > 16 * 8 * n
+        # free: too little for a download's staging (16 doubles a particle)
+        with _only_free(40 * MB):
+            got = hp.download()
+            assert hp.status()["device_bytes"] < sized
+            for k in names:
+                assert np.array_equal(got[k], want[k]), k
+            # and the pass itself still runs, in buffers of the exact sizes
+            hp.restage()
+            hp.full_pass()
+            got = hp.download(names)
+            for k in names:
+                assert np.array_equal(got[k], want[k]), k
+
+
+def test_rows_left_to_the_force_pass_survive_a_lack_of_memory():
+    """Gradients, then a download that has to find its staging in the rows' spare room, then the force on those rows."""
+    hp, _ = _crept(abi.PRECISION_FP64)
+    with hp:
+        want = hp.download()
+    hp, _ = _crept(abi.PRECISION_FP64)
+    with hp:
+        hp.restage()
+        hp.density()
+        hp.hydro_gradient_calc()
+        with _only_free(40 * MB):
+            hp.download(["rho"])
+            hp.hydro_force()
+            got = hp.download(["accel", "dudt", "vsig"])
+        for k in got:
+            assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_fp64_force_without_room_for_the_fluxes(graph):
+    """Each row then evaluates its pairs in place: the same terms in another order."""
+    n = 300_000
+    p = ics.sedov(4).params
+    with HydroPass(p) as hp:
+        hp.upload(**_uniform(n))
+        hp.full_pass()
+        want = hp.download()
+        hp.download()
+    with HydroPass(p) as hp:
+        hp.upload(**_uniform(n))
+        hp.density()
+        hp.hydro_gradient_calc()
+        hp.download()  # (its staging is held from here on)
+        with _only_free(300 * MB):  # the fluxes take 64 bytes an entry, about 800 MB
+            if graph:
+                hp.hydro_pass(graph=True, restage=True)
+                assert hp.graph_stats()["replays"] == 0
+            else:
+                hp.hydro_force()
+            got = hp.download()
+    for k in ("h", "rho", "grad_rho"):
+        assert np.array_equal(got[k], want[k]), k
+    for k in ("accel", "dudt", "vsig"):
+        scale = np.abs(want[k]).max()
+        assert np.abs(got[k] - want[k]).max() <= 1e-12 * scale, k
