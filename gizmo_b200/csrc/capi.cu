@@ -2059,7 +2059,10 @@ static int stage_inputs(gz_context *c)
     c->err = 0;
     c->err_index = -1;
     c->msg[0] = 0;
-    if (enqueue_restage(c, false)) return c->err;
+    if (enqueue_restage(c, false)) {  // the mirror or the octree is not whole
+        c->grid_valid = c->have_density = c->have_gradients = c->sym_valid = c->dens_all = false;
+        return c->err;
+    }
     c->grid_valid = true;
     c->have_density = c->have_gradients = false;
     c->sym_valid = false;
@@ -2076,6 +2079,19 @@ static int upload_from(gz_context *c, const gz_particles *in, cudaMemcpyKind kin
     cudaSetDevice(c->device);
     c->in_pending = false;  // a pipelined upload not yet restaged is superseded
     const int n = (int)in->n;
+    // A set whose buffers cannot be had, or that is refused after the size has changed, leaves the
+    // context as it was before its first upload: empty, its passes refused.
+    const bool resized = n != c->n;
+    auto nothing_held = [&] {
+        c->n = 0;
+        c->grid_valid = c->have_density = c->have_gradients = c->have_bins = c->sym_valid = c->dens_all = false;
+        return c->err;
+    };
+    auto refused = [&](const char *what) {
+        const int code = fail(c, GZ_ERR_ARG, what);
+        if (resized) nothing_held();
+        return code;
+    };
     c->n = n;
     cudaStream_t s = c->stream;
     const size_t N = (size_t)std::max(n, 1);
@@ -2083,7 +2099,7 @@ static int upload_from(gz_context *c, const gz_particles *in, cudaMemcpyKind kin
                      &c->drkern, &c->divvel, &c->rho, &c->pressure, &c->fce, &c->dudt, &c->vsig, &c->dtmass,
                      &c->dmass, &c->h_built, &c->o_mass, &c->o_u, &c->o_dt, &c->o_h, &c->o_cond, &c->dl};
     for (DevBuf *b : one)
-        if (ensure(c, *b, sizeof(double) * N)) return c->err;
+        if (ensure(c, *b, sizeof(double) * N)) return nothing_held();
     if (ensure(c, c->nvt, sizeof(double) * 6 * N) || ensure(c, c->pv, sizeof(double) * 3 * N) ||
         ensure(c, c->grad, sizeof(double) * 15 * N) || ensure(c, c->accel, sizeof(double) * 3 * N) ||
         ensure(c, c->gw, sizeof(double) * 3 * N) || ensure(c, c->fabs3, sizeof(double) * 3 * N) ||
@@ -2095,7 +2111,7 @@ static int upload_from(gz_context *c, const gz_particles *in, cudaMemcpyKind kin
         ensure(c, c->d_beg, sizeof(long long) * N) || ensure(c, c->d_end, sizeof(long long) * N) ||
         ensure(c, c->rec, std::max({sizeof(DensRec), gradient_record_bytes(0), gradient_record_bytes(1),
                                     force_record_bytes(0), force_record_bytes(1)}) * N))
-        return c->err;
+        return nothing_held();
     if (n > 0) {
         GZ_CUDA(c, cudaMemcpyAsync(c->stage3.p, in->pos, sizeof(double) * 3 * (size_t)n, kind, s));
         GZ_CUDA(c, cudaMemcpyAsync(c->o_vel.p, in->vel, sizeof(double) * 3 * (size_t)n, kind, s));
@@ -2106,16 +2122,19 @@ static int upload_from(gz_context *c, const gz_particles *in, cudaMemcpyKind kin
             else GZ_CUDA(c, cudaMemsetAsync(f.dst->p, 0, sizeof(double) * (size_t)n, s));
         }
     }
+    const bool had_bins = c->have_bins;
     c->have_bins = in->timebin != nullptr;
     if (c->have_bins) {
         if (ensure(c, c->o_timebin, sizeof(int) * N) || ensure(c, c->o_vsig, sizeof(double) * N) ||
             ensure(c, c->timebin, sizeof(int) * N) || ensure(c, c->vsig_prev, sizeof(double) * N) ||
             ensure(c, c->wakeup, sizeof(int) * N))
-            return c->err;
+            return nothing_held();
         if (kind == cudaMemcpyHostToDevice)
             for (int k = 0; k < n; k++)
-                if (in->timebin[k] < 0 || in->timebin[k] >= GZ_TIMEBINS)
-                    return fail(c, GZ_ERR_ARG, "timebin out of range");
+                if (in->timebin[k] < 0 || in->timebin[k] >= GZ_TIMEBINS) {
+                    c->have_bins = had_bins;
+                    return refused("timebin out of range");
+                }
         if (n > 0) {
             GZ_CUDA(c, cudaMemcpyAsync(c->o_timebin.p, in->timebin, sizeof(int) * (size_t)n, kind, s));
             if (in->vsig)
@@ -2127,7 +2146,7 @@ static int upload_from(gz_context *c, const gz_particles *in, cudaMemcpyKind kin
     if (!c->box_counts.empty()) {
         long long total = 0;
         for (long long k : c->box_counts) total += k;
-        if (total != n) return fail(c, GZ_ERR_ARG, "box counts do not add up to the particle count");
+        if (total != n) return refused("box counts do not add up to the particle count");
         // the box of each particle from the boxes' first particles: 8 bytes a box cross to
         // the device (a list of n box numbers filled and copied by the host took 0.6 ms of
         // an upload of 680,000 particles)
@@ -2135,7 +2154,7 @@ static int upload_from(gz_context *c, const gz_particles *in, cudaMemcpyKind kin
         std::vector<long long> first(nb);
         long long at = 0;
         for (size_t k = 0; k < nb; k++) { first[k] = at; at += c->box_counts[k]; }
-        if (ensure(c, c->box_bid, sizeof(int) * N) || ensure(c, c->box_first, sizeof(long long) * nb)) return c->err;
+        if (ensure(c, c->box_bid, sizeof(int) * N) || ensure(c, c->box_first, sizeof(long long) * nb)) return nothing_held();
         GZ_CUDA(c, cudaMemcpyAsync(c->box_first.p, first.data(), sizeof(long long) * nb, cudaMemcpyHostToDevice, s));
         if (n > 0) {
             k_box_ids<<<(n + 255) / 256, 256, 0, s>>>(n, (int)nb, ptr<long long>(c->box_first), ptr<int>(c->box_bid));
@@ -2143,7 +2162,7 @@ static int upload_from(gz_context *c, const gz_particles *in, cudaMemcpyKind kin
         }
         GZ_CUDA(c, cudaStreamSynchronize(s));  // (first is freed on return)
     }
-    if (stage_inputs(c)) return c->err;
+    if (stage_inputs(c)) return nothing_held();
     GZ_CUDA(c, cudaStreamSynchronize(s));
     return c->err;
 }

@@ -52,6 +52,11 @@ def test_a_failed_allocation_reports_cudas_own_words_and_can_be_repeated():
         with _only_free(100 * MB):
             with pytest.raises(GizmoHydroError, match="cudaMalloc of [0-9]+ bytes: out of memory"):
                 hp.upload(**big)
+        # the set is lost with its buffers: what needs one is refused, and a download has nothing to bring
+        for call in (hp.density, hp.hydro_gradient_calc, hp.hydro_force, lambda: hp.neighbors(0)):
+            with pytest.raises(GizmoHydroError) as e:
+                call()
+            assert e.value.code == abi.ERR_ORDER
         hp.upload_workload(wl)
         hp.full_pass()
         got = hp.download()
