@@ -143,7 +143,8 @@ EXPORTED_SYMBOLS = [
     "gz_neighbors", "gz_density_sums", "gz_density_sums_noalloc", "gz_kick",
     "gz_drift", "gz_set_bin_active", "gz_active_list", "gz_wakeup_bins", "gz_timestep",
     "gz_upload_device", "gz_download_device", "gz_get_tuning", "gz_set_tuning", "gz_autotune",
-    "gz_hydro_pass", "gz_graph_stats", "gz_upload_async", "gz_download_async", "gz_wait", "gz_set_boxes",
+    "gz_hydro_pass", "gz_graph_stats", "gz_force_deferred", "gz_upload_async", "gz_download_async", "gz_wait",
+    "gz_set_boxes",
 ]
 PASS_GRAPH = 1  # GZ_PASS_GRAPH
 PASS_RESTAGE = 2  # GZ_PASS_RESTAGE
@@ -199,6 +200,7 @@ def load_library(path: str | None = None) -> C.CDLL:
     lib.gz_set_bin_active.argtypes = [vp, _ip]
     lib.gz_active_list.argtypes = [vp, _ip, _ip, _ip]
     lib.gz_wakeup_bins.argtypes = [vp, _ip, C.c_int, C.c_int, _ip, _ip]
+    lib.gz_force_deferred.argtypes = [vp, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
     for name in EXPORTED_SYMBOLS:
         if name != "gz_stream":
             getattr(lib, name).restype = C.c_int

@@ -2422,6 +2422,7 @@ int gz_hydro_force(gz_context *c, const int *active, int n_active)
     long long cap = mixed ? std::max(65536ll, c->pairs_symmetric / 8) : 0;
     if (ensure(c, c->refined, sizeof(unsigned long long)) || ensure(c, c->deferred, sizeof(unsigned long long)))
         return c->err;
+    GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), c->stream));
     bool room = false;
     for (long long items : {deferred_cap(c->pairs_symmetric), 1024ll}) {  // (fewer than are deferred: the rows are scanned)
         std::vector<Need> need = {{&c->dq, sizeof(RefineItem) * (size_t)items},
@@ -2506,6 +2507,20 @@ int gz_set_boxes(gz_context *c, int n_boxes, const int64_t *counts)
         c->box_bits = 3 * ((bits + 2) / 3);  // whole octree levels
     }
     c->grid_valid = false;  // the next upload builds the grid of the boxes
+    return GZ_OK;
+}
+
+int gz_force_deferred(gz_context *c, int64_t *pairs, int64_t *room)
+{
+    if (!c || !pairs || !room) return GZ_ERR_ARG;
+    cudaSetDevice(c->device);
+    unsigned long long count = 0;
+    if (c->deferred.p) {
+        GZ_CUDA(c, cudaMemcpyAsync(&count, c->deferred.p, sizeof(count), cudaMemcpyDeviceToHost, c->stream));
+        GZ_CUDA(c, cudaStreamSynchronize(c->stream));
+    }
+    *pairs = (int64_t)count;
+    *room = (int64_t)(c->dq.bytes / sizeof(RefineItem));
     return GZ_OK;
 }
 

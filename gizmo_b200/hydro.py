@@ -245,6 +245,12 @@ class HydroPass:
         self._check(self.lib.gz_graph_stats(self._ctx, C.byref(g)))
         return {k: int(getattr(g, k)) for k, _ in abi.GzGraphInfo._fields_}
 
+    def force_deferred(self):
+        """(deferred pairs of the last force pass, room of their queue): gz_force_deferred."""
+        pairs, room = C.c_int64(), C.c_int64()
+        self._check(self.lib.gz_force_deferred(self._ctx, C.byref(pairs), C.byref(room)))
+        return pairs.value, room.value
+
     # -- walk tuning ------------------------------------------------------------
     def tuning(self) -> dict:
         t = abi.GzTuning()

@@ -223,6 +223,12 @@ typedef struct gz_graph_info {
 } gz_graph_info;
 int gz_graph_stats(gz_context *ctx, gz_graph_info *out);
 
+/* The pairs (row entries, with an active list) of the last force pass whose face
+ * the first attempt did not settle and that were evaluated by a kernel of their
+ * own, and the room of the queue they go through; when more were deferred than
+ * that, they were found by a scan of the rows. Results do not depend on the route. */
+int gz_force_deferred(gz_context *ctx, int64_t *pairs, int64_t *room);
+
 /* Copy outputs device -> host (original order). */
 int gz_download(gz_context *ctx, const gz_outputs *out);
 

@@ -41,11 +41,18 @@ def test_deferred_faces_match_the_oracle(method, mach):
         assert field_err(k, g[k], st[k].reshape(g[k].shape), 1e-3) < 1e-10, k
 
 
+def _stiff_case(method, n1):
+    """A stiff gas at Mach 2: a third of its MFM pairs is deferred (at gamma = 5/3, one in 16 at most)."""
+    wl = riemann_fallback_case(method, n1=n1, mach=2.0)
+    wl.params.gamma = 10.0
+    return wl
+
+
 @pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_MIXED], ids=["fp64", "mixed"])
 def test_more_deferred_pairs_than_the_queue_holds(precision):
-    """48^3 cells at Mach 200: over 65,536 deferred pairs, so a pass scans its marked entries; the same cells as an
+    """More pairs are deferred than the queue has room for, so a pass scans its marked entries; the same cells as an
     active list of all but one (the row entries' route), and a slice of them small enough for the queue."""
-    wl = riemann_fallback_case(abi.METHOD_MFM, n1=48, mach=200.0)
+    wl = _stiff_case(abi.METHOD_MFM, 32)
     wl.params.precision = precision
     part = np.arange(0, 2000, dtype=np.int32)
     # (an active list whose fragile pairs outgrow the mixed form's queue is refused, so only FP64 takes the long one)
@@ -55,12 +62,49 @@ def test_more_deferred_pairs_than_the_queue_holds(precision):
         hp.density()
         hp.hydro_gradient_calc()
         hp.hydro_force()
+        deferred, room = hp.force_deferred()
+        assert deferred > room >= 65536
         full = hp.download(list(FORCE))
         hp.hydro_force(part)
+        deferred, room = hp.force_deferred()
+        assert 0 < deferred <= room
         small = hp.download(list(FORCE))
         hp.hydro_force(most)
+        deferred, room = hp.force_deferred()
+        assert (deferred > room) == (precision == abi.PRECISION_FP64)
         large = hp.download(list(FORCE))
     assert np.isfinite(full["accel"]).all()
     for k in ("accel", "dudt", "vsig"):  # the same terms, summed in the rows' order in each
         assert np.array_equal(full[k][part], small[k][part]), k
         assert np.array_equal(full[k][most], large[k][most]), k
+
+
+@pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_MIXED], ids=["fp64", "mixed"])
+def test_an_overflowing_queue_in_the_graph(precision):
+    """The captured pass answers a full queue by the same scan as a plain one, and both match the oracle."""
+    wl = _stiff_case(abi.METHOD_MFM, 32)
+    wl.params.precision = precision
+    with HydroPass(wl.params) as hp:
+        hp.upload_workload(wl)
+        hp.full_pass()
+        deferred, room = hp.force_deferred()
+        assert deferred > room
+        g = hp.download()
+        hp.restage()
+        hp.hydro_pass(graph=True)
+        deferred, room = hp.force_deferred()
+        assert deferred > room
+        again = hp.download()
+        assert hp.graph_stats()["replays"] == 1 and hp.graph_stats()["fallbacks"] == 0
+    for k in g:
+        assert np.array_equal(g[k], again[k]), k
+    if precision == abi.PRECISION_MIXED:
+        return
+    st = O.new_state(wl.n, wl.inputs())
+    orc = O.Oracle(wl.params, "port")
+    for k in ("h", "num_ngb", "drkern", "divvel", "rho", "pressure", "nvt", "cond", "fce", "pvel", "grad_rho", "grad_p",
+              "grad_v"):
+        st[k][...] = g[k].reshape(st[k].shape)
+    assert orc.force(st) == 0
+    for k in FORCE:
+        assert field_err(k, g[k], st[k].reshape(g[k].shape), 1e-3) < 1e-10, k
