@@ -1125,32 +1125,77 @@ GZ_DEV void deferred_pair(const PassParams &p, const Particles &ps, const GConst
 }
 
 // The deferred pairs, one per thread over the count the pair kernel left on the
-// device. When more were deferred than the queue holds, the rows are scanned for
-// the marked entries instead and each is evaluated for itself (`all`: every
-// particle a target, no wake-up test).
+// device. When more were deferred than the queue holds, the rows are scanned for the
+// marked entries instead (`all`: every particle a target, each pair found in its lower
+// row): a warp takes 32 rows, spreads their entries over its lanes and gathers the
+// marked ones in shared memory, so that it evaluates 32 at a time here too.
 template <typename T>
 __global__ void __launch_bounds__(128) k_force_deferred(PassParams p, Particles ps, const int *__restrict__ targets,
                                                         int n_rows, Csr rows, DevStatus *st,
                                                         const ForceRec<T> *__restrict__ rec, PairFlux<T> *flux, int all,
                                                         RefineQueue q, RefineQueue dq)
 {
+    __shared__ RefineItem s_found[4][64];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
     const long long n = (long long)*dq.count;
     const GConst<T> gc = make_gconst<T>(p.gamma, p.method == 1);
-    const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const long long stride = (long long)gridDim.x * blockDim.x;
-    if (n <= dq.cap) {
-        for (long long k = first; k < n; k += stride) deferred_pair(p, ps, gc, rec, flux, dq.item[k], st, q);
-        return;
-    }
-    for (long long s = first; s < n_rows; s += stride) {
-        const int t = targets[s];
-        const long long b1 = rows.off[s + 1];
-        for (long long e = rows.off[s]; e < b1; e++) {
-            if (flux[e].valid != kDeferred) continue;
-            const int j = rows.nbr[e];
-            const RefineItem it{e, -1, t < j ? t : j, t < j ? j : t, all ? -1 : t, 0};
-            deferred_pair(p, ps, gc, rec, flux, it, st, q);
+    long long next = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    // the scan's state: the rows under way (lane k: the entries of row r0 + k), the entries seen, the pairs found
+    RefineItem *found = s_found[threadIdx.x >> 5];
+    long long r0 = next - lane - stride, beg = 0;
+    int cnt = 0, incl = 0, total = 0, base = 0, held = 0;
+    for (;;) {  // up to 32 pairs at a time, one per lane
+        RefineItem it{};
+        bool mine;
+        if (n <= dq.cap) {
+            if (next - lane >= n) break;
+            mine = next < n;
+            if (mine) it = dq.item[next];
+            next += stride;
+        } else {
+            while (held < 32) {
+                if (base >= total) {
+                    r0 += stride;
+                    if (r0 >= n_rows) break;
+                    cnt = 0;
+                    if (r0 + lane < n_rows) {
+                        const long long end = rows.off[r0 + lane + 1];
+                        beg = rows.off[r0 + lane];
+                        if (all) beg = lower_bound_row(rows.nbr, beg, end, (int)(r0 + lane) + 1);
+                        cnt = (int)(end - beg);
+                    }
+                    incl = warp_inclusive_sum(cnt);
+                    total = __shfl_sync(full, incl, 31);
+                    base = 0;
+                    continue;
+                }
+                const int f = base + lane;
+                const int k = row_of_pair(incl, f);
+                const long long e = __shfl_sync(full, beg, k) + (f - __shfl_sync(full, incl - cnt, k));
+                const bool hit = f < total && flux[e].valid == kDeferred;
+                const unsigned bal = __ballot_sync(full, hit);
+                if (hit) {
+                    const int t = targets[r0 + k], j = rows.nbr[e];
+                    found[held + __popc(bal & ((1u << lane) - 1u))] =
+                        RefineItem{e, -1, t < j ? t : j, t < j ? j : t, all ? -1 : t, 0};
+                }
+                held += __popc(bal);
+                base += 32;
+            }
+            if (held == 0) break;
+            __syncwarp();
+            mine = lane < held;
+            it = found[lane];
+            const RefineItem rest = found[32 + lane];
+            held = max(held - 32, 0);
+            __syncwarp();
+            if (lane < held) found[lane] = rest;
+            __syncwarp();
+            if (mine && all) it.a = lower_bound_row(rows.nbr, rows.off[it.j], rows.off[it.j + 1], it.i);
         }
+        if (mine) deferred_pair(p, ps, gc, rec, flux, it, st, q);
     }
 }
 

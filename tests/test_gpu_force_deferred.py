@@ -108,3 +108,29 @@ def test_an_overflowing_queue_in_the_graph(precision):
     assert orc.force(st) == 0
     for k in FORCE:
         assert field_err(k, g[k], st[k].reshape(g[k].shape), 1e-3) < 1e-10, k
+
+
+@pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_MIXED], ids=["fp64", "mixed"])
+def test_an_overflowing_queue_costs_no_more_than_its_pairs(precision):
+    """A third of the pairs evaluated twice (marked, then in full) must not take longer than half of the pass again: the
+    scan keeps a warp's lanes as busy as the queue does. (2.5 leaves room for the clocks: 1.6 in FP64 and 1.5 in the
+    mixed form, 3.3 and 2.4 with a thread a row that evaluated its marked entries one by one.)"""
+    import torch
+
+    times = []
+    for wl in (riemann_fallback_case(abi.METHOD_MFM, n1=48, mach=2.0), _stiff_case(abi.METHOD_MFM, 48)):
+        wl.params.precision = precision
+        with HydroPass(wl.params) as hp:
+            hp.upload_workload(wl)
+            hp.full_pass()
+            s = torch.cuda.ExternalStream(hp.stream)
+            ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(9)]
+            for a, b in ev:
+                a.record(s)
+                hp.hydro_force()
+                b.record(s)
+            torch.cuda.synchronize()
+            times.append(np.median([a.elapsed_time(b) for a, b in ev]))
+            deferred, room = hp.force_deferred()
+    assert deferred > room
+    assert times[1] < (2.5 if precision == abi.PRECISION_FP64 else 2.0) * times[0], times
