@@ -467,7 +467,7 @@ def run_ours(args, world, rank, local):
         kernels[name] = e
     dom = max((k for k in kernels if "achieved" in kernels[k]), key=lambda k: kernels[k]["ms_per_step"], default=None)
     kernel_names = {"density_sums": "k_density_sums<double> (FP64 shape sums of the density rows, all h iterations)",
-                    "force": "k_force_pairs<float> (MFV pair flux, each pair once)",
+                    "force": "k_force_pairs<float> and k_force_deferred<float> (MFV pair flux, each pair once)",
                     "gradients": "k_gradients<double> (least-squares gradients, FP64 in both forms)"}
     roofline = None
     if dom:

@@ -1226,9 +1226,9 @@ void launch_force(const PassParams &p, const Particles &ps, const int *targets, 
         const unsigned blocks = (unsigned)((warps + 3) / 4);
         if (all) k_force_pairs<T><<<blocks, 128, 0, s>>>(p, ps, n_targets, per_warp, rows, st, rec, flux, q, dq);
         else k_force_entries<T><<<blocks, 128, 0, s>>>(p, ps, targets, n_targets, per_warp, rows, st, rec, flux, q, dq);
-        if (ev) cudaEventRecord(ev->stop, s);
         k_force_deferred<T><<<kDeferredBlocks, 128, 0, s>>>(p, ps, targets, n_targets, rows, st, rec, flux, all ? 1 : 0,
                                                             q, dq);
+        if (ev) cudaEventRecord(ev->stop, s);
         if constexpr (sizeof(T) == sizeof(float)) force_refine(p, ps, q, flux, st, s);
         k_force_gather<T><<<(unsigned)((n_targets + 127) / 128), 128, 0, s>>>(p, ps, targets, n_targets, rows, rec, grec,
                                                                               flux, sums);

@@ -111,6 +111,31 @@ def test_an_overflowing_queue_in_the_graph(precision):
 
 
 @pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_MIXED], ids=["fp64", "mixed"])
+def test_the_force_timer_spans_the_deferred_pairs(precision):
+    """GZ_TIMER_FORCE is the time of the pair evaluations. Where many pairs are deferred it must not be that of the
+    kernel that only marks them: the rest of the stage (packing, the row sums, the writeback) is the smaller part."""
+    import torch
+
+    wl = _stiff_case(abi.METHOD_MFM, 48)
+    wl.params.precision = precision
+    with HydroPass(wl.params) as hp:
+        hp.upload_workload(wl)
+        hp.full_pass()
+        s = torch.cuda.ExternalStream(hp.stream)
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        timer, stage = [], []
+        hp.kernel_timing()
+        for _ in range(5):
+            a.record(s)
+            hp.hydro_force()
+            b.record(s)
+            torch.cuda.synchronize()
+            stage.append(a.elapsed_time(b))
+            timer.append(hp.kernel_times()["force"]["ms"])
+    assert np.median(timer) > 0.55 * np.median(stage), (timer, stage)
+
+
+@pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_MIXED], ids=["fp64", "mixed"])
 def test_an_overflowing_queue_costs_no_more_than_its_pairs(precision):
     """A third of the pairs evaluated twice (marked, then in full) must not take longer than half of the pass again: the
     scan keeps a warp's lanes as busy as the queue does. (2.5 leaves room for the clocks: 1.6 in FP64 and 1.5 in the
