@@ -4,7 +4,7 @@ fields' way back to the caller's order on both sides of the size from which scal
 import numpy as np
 import pytest
 
-from gizmo_b200 import ics
+from gizmo_b200 import abi, ics
 from gizmo_b200.hydro import GizmoHydroError, HydroPass
 from oracle import oracle as O
 
@@ -75,24 +75,64 @@ def test_box_sets_with_empty_boxes():
     assert np.array_equal(nbr, np.concatenate([na, nb + a.n]))
 
 
-@pytest.mark.parametrize("n", [1, 255, 257, 87381, (1 << 18) + 1, (1 << 20) - 1, 1 << 20])
-def test_fields_return_in_the_callers_order(n):
+COLUMNS = {"h": 1, "cond": 1, "rho": 1, "pvel": 3, "nvt": 6, "grad_rho": 3, "grad_v": 9, "accel": 3, "dudt": 1,
+           "gravwork": 3, "iters": 1}
+SHEAR = np.array([[1.0, 2.0, 3.0], [-4.0, 5.0, -6.0], [7.0, -8.0, 9.0]])
+
+
+def _untouched(n, pin=False):
+    """Output arrays in which an entry that is never written shows."""
     import torch
 
+    return {k: torch.full((n, c) if c > 1 else (n,), -1 if k == "iters" else float("nan"),
+                          dtype=torch.int32 if k == "iters" else torch.float64, pin_memory=pin)
+            for k, c in COLUMNS.items()}
+
+
+@pytest.mark.parametrize("n", [255, 257, 87381, (1 << 18) + 1, (1 << 20) - 1, 1 << 20])
+def test_fields_return_in_the_callers_order(n):
+    """The same particles uploaded in two orders: every column of every field comes back with its particle, and the
+    velocity gradients of a linear flow say which column is which."""
     rng = np.random.default_rng(n)
-    pos, h, cond = rng.random((n, 3)), rng.uniform(1e-3, 2e-3, n), rng.random(n)
     wl = ics.sedov(4)
-    names = ["h", "cond", "rho", "nvt", "grad_v", "accel", "iters"]
+    wl.params.method = abi.METHOD_MFV
+    pos = rng.random((n, 3))
+    one = np.ones(n)
+    p = dict(pos=pos, vel=(pos - 0.5) @ SHEAR.T, mass=one / n, u=rng.uniform(1, 2, n), dt=one * 2.0 ** -8,
+             h=one * (32 / (4.19 * n)) ** (1 / 3), cond=rng.random(n))
+    order = rng.permutation(n)
+    got = []
     with HydroPass(wl.params) as hp:
-        hp.upload(pos, np.zeros((n, 3)), np.ones(n), np.ones(n), np.full(n, 2.0 ** -8), h, cond)
-        out = hp.download(names)
-        pinned = {k: torch.empty(n, dtype=torch.float64, pin_memory=True) for k in ("h", "cond")}
-        hp.download_raw_async({k: v.data_ptr() for k, v in pinned.items()})
-        hp.wait()
-    assert np.array_equal(out["h"], h) and np.array_equal(out["cond"], cond)
-    assert np.array_equal(pinned["h"].numpy(), h) and np.array_equal(pinned["cond"].numpy(), cond)
-    for k in names[2:]:
-        assert not out[k].any(), k
+        for q in (p, {k: np.ascontiguousarray(v[order]) for k, v in p.items()}):
+            hp.upload(**q)
+            hp.full_pass()
+            for how in ("plain", "pipelined"):
+                out = _untouched(n, pin=how == "pipelined")
+                ptrs = {k: v.data_ptr() for k, v in out.items()}
+                if how == "plain":
+                    hp.download_raw(ptrs)
+                else:
+                    hp.download_raw_async(ptrs)
+                    hp.wait()
+                got.append({k: v.numpy().copy() for k, v in out.items()})
+    for k in COLUMNS:
+        a, same, b, same_b = (g[k] for g in got)
+        assert np.isfinite(a).all() and (a != 0).any(axis=0).all(), k
+        assert np.array_equal(a, same) and np.array_equal(b, same_b), k
+        assert np.array_equal(a[order], b), k
+    inside = (np.abs(pos - 0.5) < 0.15).all(axis=1)
+    if inside.sum() >= 100:  # (away from the periodic faces, where the flow jumps)
+        grad = np.median(got[0]["grad_v"][inside], axis=0).reshape(3, 3)
+        assert np.abs(grad - SHEAR).max() < 0.1, grad
+
+
+def test_one_particle_comes_back():
+    wl = ics.sedov(4)
+    one = np.ones(1)
+    with HydroPass(wl.params) as hp:
+        hp.upload(np.full((1, 3), 0.5), np.zeros((1, 3)), one, one, one * 2.0 ** -8, one * 0.01, one * 3.0)
+        out = hp.download(["h", "cond", "iters"])
+    assert out["h"][0] == 0.01 and out["cond"][0] == 3.0 and out["iters"][0] == 0
 
 
 def test_a_new_contexts_first_download_costs_no_more_than_its_second():
