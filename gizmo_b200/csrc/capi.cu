@@ -33,16 +33,19 @@ struct DevBuf {
 // whose h outgrows its row gets a new one at `regrow` x its new h. Every sum of
 // the iteration pays for the candidates beyond h (1.52 x as many at 1.15 h, 1.16 x
 // at 1.05 h), a row that is outgrown for one more walk of its own. Density stage
-// of 2M particles in ms, (first, regrow):
-//                     1.15,1.3  1.15,1.1  1.10,1.07  1.07,1.04  1.05,1.03  1.03,1.02
-//   Plummer, noisy h      24.4      21.4       19.6       18.6        18.2      (16.3)
-//   Plummer, h +-5%        -        14.4       13.2       12.6        12.5      (12.3)
-//   lognormal, noisy h    19.5      16.9       15.9       15.4        15.3      (14.7)
-//   lognormal, h +-5%      -        12.6       11.7       11.3        11.5      (12.0)
-// (in brackets: with the shape sums taken apart from the flow sums, seven blocks per
-// multiprocessor, where 1.05,1.03 took 17.0, 12.0, 14.9 and 11.6). Up to kSmallTargets the extra walks' latency costs
-// more than the candidates: 32,768 lattice cells at h +-5% take 0.47 ms with rows
-// that hold the whole iteration and 0.56 ms at 1.05.
+// in ms, (first, regrow):
+//                        1.15,1.3  1.15,1.1  1.10,1.07  1.07,1.04  1.05,1.03  1.03,1.02
+//   2M Plummer, noisy h      21.3      18.8       17.3       16.6       16.3       15.7
+//   2M Plummer, h +-5%       15.7      13.7       12.6       12.1       11.9       12.2
+//   2M lognormal, noisy h    18.4      15.9       15.1       14.6       14.6       14.3
+//   2M lognormal, h +-5%     12.8      12.7       11.8       11.4       11.5       12.0
+//   1M Plummer, FP64         13.9      12.2       11.5       10.9       10.5       10.2
+// Small lattice sets, whose rows at 1.15 h hold the whole iteration, lose more by the extra
+// walks' latency than by the candidates: 27,000 / 64,000 / 97,336 / 250,047 cells at h +-5%
+// 0.48 / 0.64 / 0.74 / 1.37 ms at 1.15,1.1 and 0.57 / 0.70 / 0.82 / 1.41 at 1.05,1.03.
+// Clustered ones do not: 27,000 / 64,000 / 97,336 log-normal particles 1.64 / 2.04 / 2.32
+// and 1.63 / 1.80 / 2.10 ms, Plummer ones 2.21 / 2.73 / 2.81 and 2.00 / 2.48 / 2.52.
+// kSmallTargets gives the small sets to the lattices.
 struct RowFactors {
     double first, regrow;
 };
@@ -598,9 +601,13 @@ __global__ void __launch_bounds__(256) k_zero_arrays(const ZeroArrays z)
     }
 }
 
-// The restage's gathers in one launch, for small sets: above kGatherAllMax a launch
-// per array keeps the scattered reads of one array in cache together (6.52 against
-// 5.69 ms for the restage at 256^3), below it the launches themselves cost more.
+// The restage's gathers in one launch, for small sets: in large ones a launch per array
+// keeps the scattered reads of one array in cache together, in small ones the launches
+// cost more (and the bottom-up pass of the octree is queued before the node count is
+// read). Restage of 27,000 / 110,592 lattice cells 0.20 / 0.26 ms, with a launch per array
+// 0.22 / 0.28; of 250,047 / 531,441 / 1,000,000 Plummer particles 0.34 / 0.40 / 0.54 and
+// 0.36 / 0.43 / 0.55; of 2.1M / 4.2M 0.91 / 1.70 and 0.84 / 1.42. The line is on the safe
+// side: up to a million particles the one launch is 10 to 30 us the faster.
 constexpr int kGatherAllMax = 1 << 18;
 __global__ void __launch_bounds__(256) k_gather_all(int n, const int *__restrict__ perm, const double *__restrict__ pos,
                                                     const double *__restrict__ vel, const double *__restrict__ mass,

@@ -866,10 +866,15 @@ void tree_up(int n_nodes, const int4 *node, const int *parent, const double *x, 
                                                                                        boxes);
 }
 
-// Launches for wide levels: none for sets whose widest level is a few turns of
-// the cluster; the levels that uniform and strongly clustered sets have above the
-// cluster's limit otherwise. Levels left over (deeper trees) fall to the cluster
-// again, whatever their width.
+// Launches for wide levels: none for sets whose widest level is a few turns of the
+// cluster; the levels that uniform and strongly clustered sets have above the cluster's
+// limit otherwise. Levels left over (deeper trees) fall to the cluster again, whatever
+// their width. Restage with none / five / eight launches: 27,000 and 64,000 lattice cells
+// 0.20 / 0.23 / 0.24 and 0.21 / 0.24 / 0.25 ms; Plummer sets of 68,921 particles 0.26 / 0.28 /
+// 0.29, 250,047 0.35 / 0.34 / 0.35, 531,441 0.48 / 0.42 / 0.43, a million 0.65 / 0.55 / 0.56,
+// 2.1M 1.04 / 0.84 / 0.84, 4.2M 1.77 / 1.43 / 1.41. Half the particles in a clump of 1e-5 of
+// the box, whose wide levels come after the launches' last: 700,000 / 8M particles 0.58 /
+// 2.68 ms, uniform ones 0.42 / 2.39 (a launch per level: 1.27 / 3.30 and 0.77 / 2.79).
 static int wide_levels(int n) { return n <= 65536 ? 0 : n <= (1 << 20) ? 5 : 8; }
 
 int tree_build_launches(int n) { return wide_levels(n) ? wide_levels(n) + 2 : 1; }

@@ -38,25 +38,27 @@ void walk_rows_graph(const Tree &t, const double *x, const double *y, const doub
 // warps the group-mode walk holds resident (the walk takes one warp per
 // target when a sparse list's groups would not fill them)
 long long walk_group_warps();
-// The walk's mode for n_targets targets among n_particles. Groups take 32
-// consecutive targets down the tree at once, but a short list of scattered
-// targets gives few groups, each of which walks 32 unrelated regions: one warp per
-// target is faster while the groups would fill less than a quarter of the
-// resident warps (density rows rebuilt after an h regrowth: density stage of a
-// million Plummer particles 16.65 ms, 17.5 when groups had to fill all of them,
-// 17.1 and 18.2 at a 16th and a 64th). Symmetric rows are only walked for
-// active lists, whose targets lie in the same dense regions: a 16th (1% of 2M
-// particles active: gradient stage 0.84 against 1.03 ms at a quarter, 1.02 at
-// all; 10% of 1M: 1.29 ms, 2.70 at all). While the targets themselves fill the
-// warps at most kSoloWaves times, whatever their density, one warp per target is
-// faster too: a group's walk is one serial chain of ~100 us (density stage of 4,096
-// / 9,261 / 17,576 lattice cells 0.31 / 0.39 / 0.46 ms, as groups 0.38 / 0.47 / 0.47).
+// The walk's mode for n_targets targets among n_particles. Groups take 32 consecutive
+// targets down the tree at once. One warp per target is faster
+//   - while the targets fill the resident warps at most kSoloWaves times, whatever their
+//     density: a group's walk is one serial chain of ~100 us (density stage of 9,261 /
+//     17,576 lattice cells 0.37 / 0.42 ms; 0.43 / 0.44 at one wave, 0.38 / 0.43 at eight);
+//   - for density rows of targets scattered through the set (rows rebuilt after an h
+//     regrowth), whose groups walk 32 unrelated regions, while the groups would fill less
+//     than a quarter of the resident warps: density stage of a million Plummer / 110,003
+//     log-normal particles 10.50 / 2.24 ms, 11.23 / 2.24 as long as they do not fill them
+//     all, 10.50 / 2.36 without this rule.
+// Symmetric rows are only walked for active lists; only the first rule is theirs.
+// Gradient stage of 2M log-normal particles as single targets, and as groups: the 10,000 /
+// 19,000 / 38,000 cells of the shortest timesteps 0.65 / 0.88 / 1.37 and 0.68 / 0.76 /
+// 0.83 ms, random lists of 19,000 / 25,000 / 38,000 0.85 / 0.97 / 1.24 and 1.31 / 1.23 /
+// 1.22 ms (kSoloWaves ends at 18,944).
 constexpr int kSoloWaves = 4;
 __host__ __device__ inline bool walk_one_target_per_warp(long long n_targets, long long n_particles,
                                                          long long group_warps, bool symmetric)
 {
     if (n_targets <= kSoloWaves * group_warps) return true;
-    return n_targets * 4 < n_particles && (n_targets + 31) / 32 * (symmetric ? 16 : 4) < group_warps;
+    return !symmetric && n_targets * 4 < n_particles && (n_targets + 31) / 32 * 4 < group_warps;
 }
 void walk_over_graph(const Tree &t, const double *x, const double *y, const double *z, const double *reach,
                      const int *list, const long long *off, GraphState *gs, int *nbr, DevStatus *st, int blocks,

@@ -187,8 +187,8 @@ GZ_DEV void density_row(const PassParams &p, const Particles &ps, const DensityW
 
 // Resident 128-thread blocks per multiprocessor the density sums ask of the
 // register allocator: shape and flow sums eight (at most 64 registers; density
-// stage of 2M Plummer / lognormal particles 16.4 / 14.3 ms, at six, seven and nine
-// 17.7 / 15.4, 17.0 / 14.9 and 16.7 / 14.6), all 17 sums six (at eight 58 against
+// stage of 2M Plummer / lognormal particles 16.2 / 14.5 ms, at six, seven and nine
+// 17.5 / 15.5, 16.7 / 14.9 and 16.6 / 15.0), all 17 sums six (at eight 58 against
 // 49 ms for the sums of 256^3).
 template <int WHAT> constexpr int kDensityBlocks = WHAT == kSumsAll ? 6 : 8;
 
@@ -871,12 +871,12 @@ GZ_DEV void push_refine(const RefineQueue &q, bool fragile, long long e, long lo
 
 // Resident 128-thread blocks per multiprocessor the pair kernels ask of the
 // register allocator. Every pair once: FP32 five (at most 96 registers; force
-// stage of 2M lognormal / Plummer particles 9.97 / 6.12 ms, at four, six and seven
-// 10.85 / 6.58, 10.08 / 6.11, 10.03 / 6.07), FP64 four (7.14 ms for a million
-// Plummer particles, 7.37 at three; 1.33 and 1.35 ms for 110,003 lognormal ones;
-// five 7.13 and 1.74 ms, before the rows per warp followed the size). Row entries of a subset read both sides' records
-// per lane: FP32 four (1% of 2M: 0.69 ms, 0.74 at five), FP64 three (10% of 1M:
-// 1.61 ms, 1.62 at two, 1.81 at four).
+// stage of 2M lognormal / Plummer particles 9.68 / 6.07 ms, at four, six and seven
+// 10.34 / 6.44, 9.70 / 6.00 and 9.83 / 6.06), FP64 four (a million Plummer / 110,003
+// lognormal particles 7.08 / 1.29 ms, at two, three and five 8.40 / 1.53, 7.26 /
+// 1.31 and 7.11 / 1.31). Row entries of a subset read both sides' records
+// per lane: FP32 four (1% of 2M: 0.53 ms, 0.54 at three, five and six), FP64 three
+// (10% of 1M: 1.53 ms, 1.55 at two, 1.57 at four, 1.66 at five).
 template <typename T> constexpr int kForcePairsMinBlocks = sizeof(T) == 4 ? 5 : 4;
 template <typename T> constexpr int kForceEntriesMinBlocks = sizeof(T) == 4 ? 4 : 3;
 

@@ -53,7 +53,6 @@ void density_flow_split(const PassParams &p, const Particles &ps, const DensityW
     if (w.n_todo <= 0) return;
     const unsigned blocks = (unsigned)(((long long)w.n_todo * tpt + kDensityBlock - 1) / kDensityBlock);
     switch (tpt) {
-        case 4: k_density_flow_split<double, 4><<<blocks, kDensityBlock, 0, s>>>(p, ps, w, nbr, acnt, bcnt); break;
         case 8: k_density_flow_split<double, 8><<<blocks, kDensityBlock, 0, s>>>(p, ps, w, nbr, acnt, bcnt); break;
         default: k_density_flow_split<double, 16><<<blocks, kDensityBlock, 0, s>>>(p, ps, w, nbr, acnt, bcnt); break;
     }
