@@ -165,7 +165,9 @@ int gz_set_diagnostics(gz_context *ctx, int flags);
 /* Copy inputs host -> device, sort the particles by Morton key, build the
  * octree and the sorted particle mirror. Replaces the arena acquire of
  * neighbor_loop_runner.cc:2297-2302 and the spatial-index build of
- * gpu_neighbor_list.cc:1134-1169. */
+ * gpu_neighbor_list.cc:1134-1169. An upload that fails for lack of device
+ * memory, or is refused after a change of n, leaves the context empty: its
+ * passes return GZ_ERR_ORDER until an upload succeeds. */
 int gz_upload(gz_context *ctx, const gz_particles *in);
 
 /* Rebuild the octree and the sorted mirror from the inputs already resident
