@@ -100,6 +100,7 @@ struct gz_context {
     DevBuf s_acnt, s_bcnt, s_tmp;    // symmetric rows derived from the density rows
     DevBuf pflux;                    // force pass evaluating each pair once: the flux per row entry
     std::vector<DevBuf *> in_use;    // pair buffers that make_room must not give back (Using)
+    bool roomy = false;              // the last growth of the particle buffers left the device far from full
     // symmetric rows (shared by gradients and force)
     DevBuf s_off, s_nbr, s_counts;
     long long s_nbr_cap = 0;
@@ -292,7 +293,8 @@ bool make_room(gz_context *c, const DevBuf *but)
 // evolving set creep up from step to step, and freeing and allocating these buffers in each
 // of them made a step of 64,000 cells that takes 1.6 ms take 3.5. That room costs nothing when
 // memory is short: small buffers hold 100 MB of it at most, in all, and pair buffers are given
-// back (and come back at their exact sizes) before an allocation fails.
+// back (and come back at their exact sizes) before an allocation fails. The others, whose sizes
+// follow the particle count, take it only while the device is `roomy` (upload_from).
 constexpr size_t kSmallBuffer = 4 << 20;
 bool try_ensure(gz_context *c, DevBuf &b, size_t bytes, cudaError_t *why = nullptr)
 {
@@ -300,7 +302,7 @@ bool try_ensure(gz_context *c, DevBuf &b, size_t bytes, cudaError_t *why = nullp
     const size_t exact = bytes > 0 ? bytes : 16;
     const auto pair = pair_buffers(c);
     const bool creeps = b.p && exact <= b.bytes + b.bytes / 4 &&
-                        (exact <= kSmallBuffer || std::find(pair.begin(), pair.end(), &b) != pair.end());
+                        (exact <= kSmallBuffer || c->roomy || std::find(pair.begin(), pair.end(), &b) != pair.end());
     size_t want = creeps ? exact + exact / 4 : exact;
     release(b);
     cudaError_t e = cudaMalloc(&b.p, want);
@@ -2100,6 +2102,19 @@ static int upload_from(gz_context *c, const gz_particles *in, cudaMemcpyKind kin
         return code;
     };
     c->n = n;
+    const size_t held = c->x.bytes / sizeof(double);
+    if ((size_t)n > held) {
+        // A set that creeps up (a rank's share of an evolving one) would have every buffer allocated
+        // anew at each growth: with 0.1% more particles each upload, 28 / 42 ms an upload of 200,000 /
+        // 1,000,000 particles and as much again in the passes, 0.4 / 0.7 ms with room to grow. The
+        // particle buffers, which are held for good, take it only while twice all that a pass of
+        // the set can ask for is free: its records, and rows of twice the wanted neighbours with
+        // their fluxes, queues and scratch.
+        const double later = 2.0 * n * (2048.0 + 2.0 * c->prm.des_num_ngb * (pair_flux_bytes(0) + 48.0));
+        size_t free_bytes = 0, total = 0;
+        c->roomy = (size_t)n <= held + held / 4 && cudaMemGetInfo(&free_bytes, &total) == cudaSuccess &&
+                   (double)free_bytes >= later;
+    }
     cudaStream_t s = c->stream;
     const size_t N = (size_t)std::max(n, 1);
     DevBuf *one[] = {&c->x, &c->y, &c->z, &c->vx, &c->vy, &c->vz, &c->m, &c->u, &c->dt, &c->h, &c->cond, &c->num_ngb,

@@ -149,3 +149,22 @@ def test_fp64_force_without_room_for_the_fluxes(graph):
     for k in ("accel", "dudt", "vsig"):
         scale = np.abs(want[k]).max()
         assert np.abs(got[k] - want[k]).max() <= 1e-12 * scale, k
+
+
+def test_a_set_that_creeps_up_is_not_allocated_anew_each_time():
+    """Far from the device's limit; near it the buffers keep to their exact sizes."""
+    p = ics.sedov(4).params
+    n = 300_000
+    a = _uniform(n + 40)
+    part = lambda k: {f: v[:k] for f, v in a.items()}  # noqa: E731
+    sizes = {}
+    for where in ("roomy", "tight"):
+        with HydroPass(p) as hp, _only_free(2000 * MB) if where == "tight" else contextlib.nullcontext():
+            sizes[where] = []
+            for k in (n, n + 10, n + 20, n + 30, n + 40):
+                hp.upload(**part(k))
+                hp.density()
+                sizes[where].append(hp.status()["device_bytes"])
+    assert sizes["roomy"][1] > 1.1 * sizes["roomy"][0]
+    assert len(set(sizes["roomy"][1:])) == 1, sizes
+    assert sizes["tight"][4] < 1.05 * sizes["tight"][0], sizes
