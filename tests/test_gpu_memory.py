@@ -14,20 +14,15 @@ MB = 1 << 20
 
 @contextlib.contextmanager
 def _only_free(nbytes):
-    """All but about nbytes of the device's memory taken, in blocks, while the context is open."""
+    """All of the device's memory but nbytes, and 12 MB at most beyond, taken while the context is open. (The caching
+    allocator takes exact multiples of 2 MB from the device for what is larger than 10 MB, 20 MB for what is smaller.)"""
     import torch
 
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     held = []
-    block = 1 << 36
-    while block >= 2 * MB:
-        while torch.cuda.mem_get_info()[0] >= nbytes + block:
-            try:
-                held.append(torch.empty(block, dtype=torch.uint8, device="cuda"))
-            except torch.cuda.OutOfMemoryError:
-                break
-        block //= 2
+    while (excess := torch.cuda.mem_get_info()[0] - nbytes) >= 12 * MB:
+        held.append(torch.empty(min(excess, 1 << 36) // (2 * MB) * 2 * MB, dtype=torch.uint8, device="cuda"))
     try:
         yield
     finally:
@@ -149,6 +144,32 @@ def test_fp64_force_without_room_for_the_fluxes(graph):
     for k in ("accel", "dudt", "vsig"):
         scale = np.abs(want[k]).max()
         assert np.abs(got[k] - want[k]).max() <= 1e-12 * scale, k
+
+
+def test_mixed_force_with_room_for_the_fluxes_only():
+    """The queue of the deferred pairs then has room for a few of them, and the rows are scanned for the others."""
+    n = 600_000
+    q = _uniform(n)
+    q["vel"] = np.random.default_rng(2).standard_normal((n, 3)) * 2.0
+    p = ics.sedov(4, precision=abi.PRECISION_MIXED).params
+    got, names = {}, ["accel", "dudt", "vsig"]
+    for where in ("roomy", "tight"):
+        with HydroPass(p) as hp:
+            hp.upload(**q)
+            hp.density()
+            hp.hydro_gradient_calc()
+            hp.download(["h"])  # (its staging is held from here on)
+            pairs = hp.status()["pairs_symmetric"]
+            # fluxes 32 bytes an entry, the refine queue 32 for one in 8, the deferred pairs' queue 32 for one in 32;
+            # the rows' scratch, 4 an entry, is given back for them
+            with _only_free((32 + 4 - 4) * pairs + 6 * MB) if where == "tight" else contextlib.nullcontext():
+                assert pairs > 16 * MB
+                hp.hydro_force()
+                deferred, room = hp.force_deferred()
+                got[where] = hp.download(names)
+            assert deferred > 1024 and (room == 1024) == (where == "tight"), (where, deferred, room)
+    for k in names:
+        assert np.array_equal(got["tight"][k], got["roomy"][k]), k
 
 
 def test_a_set_that_creeps_up_is_not_allocated_anew_each_time():
