@@ -2683,14 +2683,17 @@ static int download_to(gz_context *c, const gz_outputs *o, bool to_device)
         }
         scatter_fields(c, f, first, last, s, at);
         GZ_CUDA(c, cudaGetLastError());
-        if (used <= kPinnedBytes && pinned_buffer(c, used) && host_writable(f, first, last)) {
+        if (used <= kPinnedBytes && pinned_buffer(c, used)) {
             GZ_CUDA(c, cudaMemcpyAsync(c->pinned, c->dl.p, used, cudaMemcpyDeviceToHost, s));
+            const bool mine = host_writable(f, first, last);  // (looked up while the copy is under way)
             GZ_CUDA(c, cudaStreamSynchronize(s));
-            for (size_t i = first; i < last; i++)
-                memcpy(f[i].dst, (char *)c->pinned + ((char *)at[i - first] - (char *)c->dl.p),
-                       (size_t)f[i].bytes * f[i].k * n);
-            first = last;
-            continue;
+            if (mine) {
+                for (size_t i = first; i < last; i++)
+                    memcpy(f[i].dst, (char *)c->pinned + ((char *)at[i - first] - (char *)c->dl.p),
+                           (size_t)f[i].bytes * f[i].k * n);
+                first = last;
+                continue;
+            }
         }
         for (size_t i = first; i < last; i++)
             GZ_CUDA(c, cudaMemcpyAsync(f[i].dst, at[i - first], (size_t)f[i].bytes * f[i].k * n, cudaMemcpyDeviceToHost, s));
