@@ -288,8 +288,8 @@ bool make_room(gz_context *c, const DevBuf *but)
 // had. (A lack of memory is cleared from the runtime; any other answer, an earlier fault
 // among them, is left there.)
 //
-// Buffers have the size that was asked for, but one that has to grow by less than a quarter
-// takes a quarter more than asked if it is a pair buffer or small: the row totals of an
+// Buffers have the size that was asked for, but a small one that has to grow, and a pair buffer
+// that has to grow by less than a quarter, take a quarter more than asked: the row totals of an
 // evolving set creep up from step to step, and freeing and allocating these buffers in each
 // of them made a step of 64,000 cells that takes 1.6 ms take 3.5. That room costs nothing when
 // memory is short: small buffers hold 100 MB of it at most, in all, and pair buffers are given
@@ -301,9 +301,9 @@ bool try_ensure(gz_context *c, DevBuf &b, size_t bytes, cudaError_t *why = nullp
     if (b.bytes >= bytes && b.p) return true;
     const size_t exact = bytes > 0 ? bytes : 16;
     const auto pair = pair_buffers(c);
-    const bool creeps = b.p && exact <= b.bytes + b.bytes / 4 &&
-                        (exact <= kSmallBuffer || c->roomy || std::find(pair.begin(), pair.end(), &b) != pair.end());
-    size_t want = creeps ? exact + exact / 4 : exact;
+    const bool creeps = exact <= b.bytes + b.bytes / 4 &&
+                        (c->roomy || std::find(pair.begin(), pair.end(), &b) != pair.end());
+    size_t want = b.p && (creeps || exact <= kSmallBuffer) ? exact + exact / 4 : exact;
     release(b);
     cudaError_t e = cudaMalloc(&b.p, want);
     if (e == cudaErrorMemoryAllocation && want > exact) {
@@ -2444,7 +2444,6 @@ int gz_hydro_force(gz_context *c, const int *active, int n_active)
     long long cap = mixed ? std::max(65536ll, c->pairs_symmetric / 8) : 0;
     if (ensure(c, c->refined, sizeof(unsigned long long)) || ensure(c, c->deferred, sizeof(unsigned long long)))
         return c->err;
-    GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), c->stream));
     bool room = false;
     for (long long items : {deferred_cap(c->pairs_symmetric), 1024ll}) {  // (fewer than are deferred: the rows are scanned)
         std::vector<Need> need = {{&c->dq, sizeof(RefineItem) * (size_t)items},
@@ -2453,6 +2452,7 @@ int gz_hydro_force(gz_context *c, const int *active, int n_active)
         if ((room = ensure_together(c, need))) break;
     }
     void *flux = room ? c->pflux.p : nullptr;
+    if (!flux) GZ_CUDA(c, cudaMemsetAsync(c->deferred.p, 0, sizeof(unsigned long long), c->stream));  // none is deferred
     if (mixed && !room) return fail(c, GZ_ERR_CAPACITY, "mixed-form force pass: no room for the pair fluxes");
     Using use(c, {&c->pflux, &c->dq, &c->s_nbr});
     const Csr rows{ptr<long long>(c->s_off), ptr<int>(c->s_nbr)};
